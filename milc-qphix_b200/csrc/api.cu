@@ -108,6 +108,7 @@ void init_context(QPHIX_layout_t *layout)
     QB_CUDA(cudaMalloc(&c.d_scalars, sizeof(double) * 64));
     QB_CUDA(cudaMalloc(&c.d_err, sizeof(int)));
     QB_CUDA(cudaMemset(c.d_err, 0, sizeof(int)));
+    QB_CUDA(cudaMalloc(&c.d_slots, solver_loop_slot_bytes()));
     QB_CUDA(cudaMallocHost(&c.h_scalars, sizeof(double) * 64));
     for (int i = 0; i < 2; ++i) {
         QB_CUDA(cudaEventCreate(&c.ev_solve[i]));
@@ -132,6 +133,8 @@ void finalize_context()
     cudaFree(c.d_scalars);
     cudaFree(c.d_err);
     c.d_err = nullptr;
+    cudaFree(c.d_slots);
+    c.d_slots = nullptr;
     cudaFreeHost(c.h_scalars);
     for (int i = 0; i < 2; ++i) {
         cudaEventDestroy(c.ev_solve[i]);
@@ -384,6 +387,28 @@ const LinkSet &single_inner_links(QPHIX_D3_FermionLinksAsqtad *H)
     return H->sloppy_recon.valid ? H->sloppy_recon : single_links(H);
 }
 
+// Whether the handle's backward links are its forward links shifted
+// (LinkSet::mirrored), asked once per handle (its links never change) and
+// only where the resident solver loop would use the answer; the derived
+// copies inherit it.
+template <typename FL>
+void note_mirrored(FL *H)
+{
+    Context &c = ctx();
+    if (c.halo.on) return;
+    std::vector<LinkSet *> sets{&H->links, &H->sloppy_half};
+    if constexpr (std::is_same<FL, QPHIX_D3_FermionLinksAsqtad>::value) {
+        sets.push_back(&H->sloppy_single);
+        sets.push_back(&H->sloppy_recon);
+    }
+    bool wanted = false;
+    for (LinkSet *s : sets) wanted = wanted || (s->valid && loop_wants_mirrored(*s, c.g.vh));
+    if (!wanted) return;
+    if (H->links.mirrored < 0)
+        H->links.mirrored = links_mirrored(H->links, c.launch(), static_cast<int *>(c.d_slots)) ? 1 : 0;
+    for (LinkSet *s : sets) s->mirrored = H->links.mirrored;
+}
+
 bool refine_batched_env()
 {
     const char *e = std::getenv("QPHIX_B200_MS_REFINE");
@@ -536,13 +561,16 @@ int asqtad_invert(QPHIX_info_t *info, typename Api<Real>::FL *H, QPHIX_invert_ar
         QB_CUDA(cudaEventRecord(c.ev_solve[0], c.stream));
         if constexpr (std::is_same<Real, double>::value) {
             if (c.inner_mode == QPHIX_B200_PREC_DOUBLE) {
+                note_mirrored(H);
                 iters = cg_reference(Prec::Double, H->links, a);
             } else {
                 const SloppyCfg s = sloppy_cfg(H, c.inner_mode);
+                note_mirrored(H);
                 iters = cg_mixed(s.vec, H->links, *s.links, s.up, a);
                 c.stats.links_compressed = s.links->recon;
             }
         } else {
+            note_mirrored(H);
             iters = cg_reference(Prec::Single, H->links, a);
         }
         QB_CUDA(cudaEventRecord(c.ev_solve[1], c.stream));
@@ -589,6 +617,7 @@ int asqtad_invert_multi(QPHIX_info_t *info, typename Api<Real>::FL *H, QPHIX_inv
         QB_CUDA(cudaEventRecord(c.ev_solve[0], c.stream));
         if constexpr (std::is_same<Real, double>::value) {
             if (c.inner_mode == QPHIX_B200_PREC_DOUBLE) {
+                note_mirrored(H);
                 iters = multishift_reference(Prec::Double, H->links, a);
             } else {
                 const SloppyCfg s = sloppy_cfg(H, c.inner_mode);
@@ -609,10 +638,12 @@ int asqtad_invert_multi(QPHIX_info_t *info, typename Api<Real>::FL *H, QPHIX_inv
                 if (rs == "half-links") rop = {Prec::Single, &half_links(H), &single_inner_links(H)};
                 else if (rs == "half") rop = {Prec::Half, &half_links(H), &single_inner_links(H)};
                 else if (rs != "single") throw Error("QPHIX_B200_MS_REFINE_STORAGE: single, half-links or half");
+                note_mirrored(H);
                 iters = multishift_mixed(s.vec, H->links, *s.links, s.up, a, l32, &rop);
                 c.stats.links_compressed = s.links->recon;
             }
         } else {
+            note_mirrored(H);
             iters = multishift_reference(Prec::Single, H->links, a);
         }
         QB_CUDA(cudaEventRecord(c.ev_solve[1], c.stream));

@@ -13,6 +13,7 @@
 
 #include "device_common.cuh"
 #include "halo.h"
+#include "solver_steps.cuh"
 
 namespace qb {
 
@@ -113,36 +114,6 @@ k_cg_restart(VecView<S> ttt, VecView<S> x, VecView<S> b, VecView<S> r, VecView<S
 }
 
 // --------------------------------------------------------- CG iteration --
-// calc_rsq2 (ks_d_congrad_fn.cpp:131-147): x += a p; r += a ttt; rsq = |r|^2
-// followed by the scalar bookkeeping of :543-566 and the completion test at
-// the top of the loop (:360-363), evaluated on the device.
-// V: sites of the whole lattice (relative_residue divides by the global
-// volume, ks_blas_utils_c.cpp:148)
-struct FinCgUpdate {
-    SolverState *st;
-    int gate;
-    bool relres;
-    double V;
-    __device__ void operator()(const double *t) const
-    {
-        const int single = st->prec_single;
-        const double oldrsq = st->rsq;
-        const double rsq = t[0];
-        st->oldrsq = oldrsq;
-        st->rsq = rsq;
-        double relrsq = st->relrsq;
-        if (relres) relrsq = round_to(sqrt(2.0 * t[1] / V), single);
-        st->relrsq = relrsq;
-        st->size_r = round_to(rsq, single) / st->source_norm;
-        st->size_relr = round_to(relrsq, single);
-        st->b = round_to(round_to(rsq, single) / oldrsq, single);
-        const bool conv = (st->rsqmin <= 0 || st->rsqmin > st->size_r) &&
-                          (st->relrsqmin <= 0 || st->relrsqmin > st->size_relr);
-        if (!isfinite(rsq) && !st->error) st->error = 1;  // non-finite residual: breakdown
-        if ((st->iteration % st->niter == 0) || conv || st->error || run_guard(st)) stop_run(st, gate);
-    }
-};
-
 template <typename S>
 __global__ void __launch_bounds__(kBlock)
 k_cg_update(VecView<S> x, VecView<S> pv, VecView<S> r, VecView<S> ttt, SolverState *st,
@@ -190,38 +161,6 @@ __global__ void __launch_bounds__(kBlock) k_cg_axpy(VecView<S> r, VecView<S> pv,
     for (int i = 0; i < 6; ++i) p[i] = rv[i] + b * p[i];
     pv.store(j, p);
 }
-
-// end of an inner iteration of the mixed CG (one thread): b, and whether
-// to stop for a reliable update
-__device__ __forceinline__ void mx_finish(SolverState *st, double rsq, int gate, double delta2)
-{
-    const double oldrsq = st->rsq;
-    st->oldrsq = oldrsq;
-    st->rsq = rsq;
-    st->b = rsq / oldrsq;
-    bool stalled = false;
-    if (rsq < st->ru_best) {
-        st->ru_best = rsq;
-        st->ru_best_iter = st->iteration;
-    } else if (st->ru_stall_window > 0 && st->iteration - st->ru_best_iter >= st->ru_stall_window) {
-        stalled = true;
-        st->ru_stalled = 1;
-    }
-    if (!isfinite(rsq) && !st->error) st->error = 1;  // non-finite residual: breakdown
-    const bool ru = (rsq < delta2 * st->rsq_ru) || (rsq <= st->rsqstop) || stalled ||
-                    (st->iteration >= st->max_cg) || st->error || run_guard(st);
-    if (ru) {
-        st->skip_axpy = 1;  // this iteration's p update waits for the true residual
-        stop_run(st, gate);
-    }
-}
-
-struct FinMx {
-    SolverState *st;
-    int gate;
-    double delta2;
-    __device__ void operator()(const double *t) const { mx_finish(st, t[0], gate, delta2); }
-};
 
 // ------------------------------------------- flat vectorised p / x, r updates --
 // In FP32 and FP64 a parity block is one contiguous array of 6 Vh reals
@@ -305,72 +244,6 @@ k_mx_update_flat(typename Wide<R>::type *x, const typename Wide<R>::type *p, typ
 }
 
 // ------------------------------------------------------------ multi-shift --
-// calc_rsq2 (ks_multicg_offset.cpp:124-140) + the convergence test (:520)
-// + the alpha recurrences (:587-598), evaluated on the device.
-struct FinMsResidual {
-    SolverState *st;
-    int gate;
-    // one warp: lane k updates shifts k, k + 32, ... (per-shift arithmetic
-    // as in the sequential form)
-    static constexpr bool kWarp = true;
-    __device__ void operator()(const double *t, int lane) const
-    {
-        const int single = st->prec_single;
-        const double rsq = t[0];
-        int done = 0;
-        if (lane == 0) {
-            const double oldrsq = st->rsq;
-            st->oldrsq = oldrsq;
-            st->rsq = rsq;
-            if (!isfinite(rsq) && !st->error) st->error = 1;  // non-finite residual: breakdown
-            if (st->error) {  // (or a zero p.Ap in the Dslash kernel before)
-                stop_run(st, gate);
-                done = 1;
-            } else if (rsq <= st->rsqstop) {
-                st->converged = 1;
-                stop_run(st, gate);
-                done = 1;
-            } else {
-                st->alpha[st->j_low] = round_to(rsq / oldrsq, single);
-            }
-        }
-        if (__shfl_sync(0xffffffffu, done, 0)) return;
-        __syncwarp();
-        const int jl = st->j_low;
-        const int nn = st->num_now;
-        const double a_jl = st->alpha[jl], b_jl = st->beta_i[jl];
-        const int it = st->iteration;
-        const double stop = st->shift_stop;
-        for (int k = lane; k < nn; k += 32) {
-            if (k == jl) continue;
-            const double zb = round_to(st->zeta_i[k] * b_jl, single);
-            if (zb != 0.0)
-                st->alpha[k] = round_to(round_to(round_to(a_jl * st->zeta_ip1[k], single) * st->beta_i[k], single) / zb,
-                                        single);
-            else { st->alpha[k] = 0.0; st->finished[k] = 1; }
-            if (stop > 0.0 && st->shift_done_at[k] == INT_MAX) {
-                const double z = st->zeta_ip1[k];
-                if (z * z * rsq <= stop) st->shift_done_at[k] = it;
-            }
-        }
-        __syncwarp();
-        if (lane == 0) {
-            // the iteration completes (its vector updates are not gated off);
-            // the host then replaces r by the FP64 residual of the base shift
-            if (st->ms_delta2 > 0.0 && rsq < st->ms_delta2 * st->rsq_ru) {
-                st->ms_ru = 1;
-                stop_run(st, gate);
-            }
-            // deferred shift updates: this iteration takes the segment's last slot
-            if (st->ms_seg_cap > 0 && st->iteration - st->ms_seg_start >= st->ms_seg_cap) {
-                st->ms_seg_full = 1;
-                stop_run(st, gate);
-            }
-            if (st->iteration >= st->max_cg || run_guard(st)) stop_run(st, gate);
-        }
-    }
-};
-
 template <typename S>
 __global__ void __launch_bounds__(kBlock)
 k_ms_residual(VecView<S> r, VecView<S> ttt, SolverState *st, double *partials, int gate, SolverState *split)

@@ -229,6 +229,7 @@ void free_links(LinkSet &ls)
         ls.lam[cb] = nullptr;
     }
     ls.valid = false;
+    ls.mirrored = -1;
     ls.recon = 0;
 }
 

@@ -102,6 +102,7 @@ struct Context {
     std::string last_error;
 
     int *d_err = nullptr;            // kernel failure word (bounded waits)
+    void *d_slots = nullptr;         // barrier slots of the resident solver loop
     HostStaging staging;             // made on the first large pageable upload
     Halo halo;                       // domain decomposition along t (halo.h)
     int global_dims[4] = {0, 0, 0, 0};  // the whole lattice (dims: this GPU's slab)

@@ -269,6 +269,24 @@ template <> struct LinkView<Recon13> : ReconLinks {
     }
 };
 
+// the links of output parity cb
+template <typename SL>
+inline LinkView<SL> link_view(const LinkSet &ls, int cb, int vh)
+{
+    if constexpr (std::is_same<SL, __half>::value)
+        return LinkView<__half>{static_cast<const int4 *>(ls.blk[cb]), vh, ls.link_max[0] / 32767.0f,
+                                ls.link_max[1] / 32767.0f};
+    else if constexpr (std::is_same<SL, float>::value)
+        return LinkView<float>{static_cast<const float4 *>(ls.blk[cb]), vh};
+    else if constexpr (std::is_same<SL, Recon12>::value)
+        return LinkView<Recon12>{{static_cast<const float4 *>(ls.blk[cb]), vh},
+                                 static_cast<const unsigned *>(ls.sign[cb]), ls.recon_scale};
+    else if constexpr (std::is_same<SL, Recon13>::value)
+        return LinkView<Recon13>{{static_cast<const float4 *>(ls.blk[cb]), vh}, static_cast<const float4 *>(ls.lam[cb])};
+    else
+        return LinkView<double>{static_cast<const double2 *>(ls.blk[cb]), vh};
+}
+
 // ------------------------------------------------------------------ SU(3) --
 // acc += U v
 template <typename A>
@@ -297,6 +315,43 @@ __device__ __forceinline__ void mv_adj_sub(A acc[6], const A u[18], const A v[6]
             const A ur = u[6 * c + 2 * r], ui = u[6 * c + 2 * r + 1];
             acc[2 * r] -= ur * v[2 * c] + ui * v[2 * c + 1];
             acc[2 * r + 1] -= ur * v[2 * c + 1] - ui * v[2 * c];
+        }
+    }
+}
+
+__device__ __forceinline__ double fma_(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float fma_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+
+// The same as chains of fused multiply-adds: two instructions per pair of real
+// products, where acc += a * b - c * d compiles to three (one rounding less
+// per term).  For kernels that the instruction issue bounds.
+template <typename A>
+__device__ __forceinline__ void mv_add_fma(A acc[6], const A u[18], const A v[6])
+{
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const A ur = u[6 * r + 2 * c], ui = u[6 * r + 2 * c + 1];
+            acc[2 * r] = fma_(ur, v[2 * c], acc[2 * r]);
+            acc[2 * r] = fma_(-ui, v[2 * c + 1], acc[2 * r]);
+            acc[2 * r + 1] = fma_(ur, v[2 * c + 1], acc[2 * r + 1]);
+            acc[2 * r + 1] = fma_(ui, v[2 * c], acc[2 * r + 1]);
+        }
+    }
+}
+template <typename A>
+__device__ __forceinline__ void mv_adj_sub_fma(A acc[6], const A u[18], const A v[6])
+{
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const A ur = u[6 * c + 2 * r], ui = u[6 * c + 2 * r + 1];
+            acc[2 * r] = fma_(-ur, v[2 * c], acc[2 * r]);
+            acc[2 * r] = fma_(-ui, v[2 * c + 1], acc[2 * r]);
+            acc[2 * r + 1] = fma_(-ur, v[2 * c + 1], acc[2 * r + 1]);
+            acc[2 * r + 1] = fma_(ui, v[2 * c], acc[2 * r + 1]);
         }
     }
 }

@@ -22,6 +22,7 @@
 
 #include "device_common.cuh"
 #include "halo.h"
+#include "solver_steps.cuh"
 #include "tunecache.h"
 
 namespace qb {
@@ -221,79 +222,6 @@ template <> struct MinBlocks<float, Recon12> { static constexpr int value = 3; }
 template <> struct MinBlocks<float, Recon13> { static constexpr int value = 3; };
 template <> struct MinBlocks<float, __half> { static constexpr int value = 3; };
 template <> struct MinBlocks<__half, __half> { static constexpr int value = 3; };
-
-// Scalar step after p.(M^dag M p) is known, run by one warp of the last
-// block of the reduction: CG (mode 0) a = -rsq/pkp in lane 0; multi-shift
-// (mode 1) the shift recurrences, lane k handling shifts k, k + 32, ...
-// (each shift's arithmetic is the sequential one, so the results do not
-// depend on the lane split; one thread walking the shifts through device
-// memory took ~10 us per iteration at 12 shifts).
-// A zero or non-finite p.(M p) is a breakdown (M is positive definite for
-// m > 0; the reference divides by it unchecked, ks_d_congrad_fn.cpp:511):
-// the step is set to zero, st->error = 2 and the update kernel that follows
-// ends the device run, so the host returns QPHIX_FAIL.
-struct FinMdagm {
-    SolverState *st;
-    int mode;
-    static constexpr bool kWarp = true;
-    __device__ void operator()(const double *t, int lane) const
-    {
-        const double pkp = t[0];
-        int done = 0;
-        if (lane == 0) {
-            st->pkp = pkp;
-            st->iteration += 1;
-            if (!(pkp != 0.0) || !isfinite(pkp)) {
-                st->error = 2;
-                st->a = 0.0;
-                done = 1;
-            } else if (mode == 0) {
-                st->a = round_to(-st->rsq / pkp, st->prec_single);
-                done = 1;
-            }
-        }
-        if (__shfl_sync(0xffffffffu, done, 0)) return;
-        // multi-shift scalar recurrences (ks_multicg_offset.cpp:475-496);
-        // the values of the previous iteration are scrolled first
-        // (:617-622), which the reference does at the end of that iteration
-        const int single = st->prec_single;
-        const int jl = st->j_low;
-        const int nn = st->num_now;
-        if (!st->first_iter) {
-            for (int k = lane; k < nn; k += 32) {
-                st->beta_im1[k] = st->beta_i[k];
-                st->zeta_im1[k] = st->zeta_i[k];
-                st->zeta_i[k] = st->zeta_ip1[k];
-            }
-        }
-        __syncwarp();
-        if (lane == 0) {
-            st->first_iter = 0;
-            st->beta_i[jl] = round_to(-st->rsq / pkp, single);
-            st->zeta_ip1[jl] = 1.0;
-        }
-        __syncwarp();
-        const double b_jl = st->beta_i[jl], a_jl = st->alpha[jl], bm1_jl = st->beta_im1[jl];
-        for (int k = lane; k < nn; k += 32) {
-            if (k == jl) continue;
-            const double zi = st->zeta_i[k], zim1 = st->zeta_im1[k];
-            double z = round_to(round_to(zi * zim1, single) * bm1_jl, single);
-            const double c1 = round_to(round_to(b_jl * a_jl, single) * round_to(zim1 - zi, single), single);
-            const double c2 =
-                round_to(round_to(zim1 * bm1_jl, single) * (1.0 + round_to(st->shifts[k] * b_jl, single)), single);
-            const double den = round_to(c1 + c2, single);
-            if (den != 0.0) z = round_to(z / den, single);
-            else { z = 0.0; st->finished[k] = 1; }
-            st->zeta_ip1[k] = z;
-            if (zi != 0.0)
-                st->beta_i[k] = round_to(round_to(b_jl * z, single) / zi, single);
-            else { st->zeta_ip1[k] = 0.0; st->beta_i[k] = 0.0; st->finished[k] = 1; }
-        }
-        __syncwarp();
-        // the last active shift leaves the recurrence once it has finished
-        if (lane == 0 && nn - 1 > jl && st->finished[nn - 1] == 1) st->num_now = nn - 1;
-    }
-};
 
 template <typename SV, typename SL>
 __global__ void __launch_bounds__(kBlock, MinBlocks<SV, SL>::value) k_dslash(DslashArgs<SV, SL> a, const SolverState *st, int gate)
@@ -708,20 +636,7 @@ static DslashArgs<SV, SL> make_args(const Launch &L, VecBlock out, VecBlock in, 
     DslashArgs<SV, SL> a;
     a.out = view<SV>(out, L.g->vh);
     a.in = view<SV>(in, L.g->vh);
-    if constexpr (std::is_same<SL, __half>::value) {
-        a.links = LinkView<__half>{static_cast<const int4 *>(ls.blk[cb]), L.g->vh,
-                                   ls.link_max[0] / 32767.0f, ls.link_max[1] / 32767.0f};
-    } else if constexpr (std::is_same<SL, float>::value) {
-        a.links = LinkView<float>{static_cast<const float4 *>(ls.blk[cb]), L.g->vh};
-    } else if constexpr (std::is_same<SL, Recon12>::value) {
-        a.links = LinkView<Recon12>{{static_cast<const float4 *>(ls.blk[cb]), L.g->vh},
-                                    static_cast<const unsigned *>(ls.sign[cb]), ls.recon_scale};
-    } else if constexpr (std::is_same<SL, Recon13>::value) {
-        a.links = LinkView<Recon13>{{static_cast<const float4 *>(ls.blk[cb]), L.g->vh},
-                                    static_cast<const float4 *>(ls.lam[cb])};
-    } else {
-        a.links = LinkView<double>{static_cast<const double2 *>(ls.blk[cb]), L.g->vh};
-    }
+    a.links = link_view<SL>(ls, cb, L.g->vh);
     a.g = *L.g;
     a.cb = cb;
     return a;
@@ -790,6 +705,8 @@ static int forced_variant()
     }
     return g_forced;
 }
+
+bool dslash_variant_forced() { return forced_variant() >= 0; }
 
 void set_forced_variant(int v)
 {

@@ -75,6 +75,7 @@ struct LinkSet {
     float link_max[2] = {0.f, 0.f};     // half only: fixed-point range of fat / Naik links
     Prec prec = Prec::Double;           // storage precision of the blocks
     bool valid = false;
+    int mirrored = -1;  // links_mirrored() of the set it was made from; -1: not asked yet
     // FP32 with compressed Naik links (recon 1: 12-real, 2: 13-real): per
     // direction the fat pair (9 float4) and rows 0-1 of the Naik pair (6
     // float4); row 2 is rebuilt as lambda * conj(row0 x row1) with
@@ -265,6 +266,41 @@ void ms_coef(const Launch &L, const MsHistEntry *hist_s, int m, int n, int j_low
 // (x, p0, p: device arrays indexed by shift)
 void ms_flush(const Launch &L, VecBlock hist, int m, const double *coef, const int *jobs, int njobs,
               VecBlock *x, const VecBlock *p0, VecBlock *p);
+
+// Resident solver loop (loop.cu): the iterations of one solver phase in one
+// cooperative launch.  `q` names the vectors and scalars that the phase's
+// kernels would get; the device state must be on the GPU with stop_at =
+// INT_MAX, use_cond = 0 and err = nullptr.  False when the phase has no
+// resident form (the caller then runs its kernels one by one).
+enum LoopMode : int {
+    kLoopCg = 0,       // dslash, mdagm, cg_update (no relative residue), cg_axpy
+    kLoopMx = 1,       // dslash, mdagm, mx_update, cg_axpy
+    kLoopMs = 2,       // dslash, mdagm, ms_residual, ms_update (x in the vectors' precision)
+    kLoopMsDefer = 3,  // dslash, mdagm, ms_residual, ms_defer
+};
+struct LoopRun {
+    int mode = kLoopCg;
+    const LinkSet *links = nullptr;
+    int parity = 0;
+    VecBlock p, tmp, ttt, r, x;
+    double m4 = 0, delta2 = 0;
+    SolverState *st = nullptr;
+    void *slots = nullptr;  // solver_loop_slot_bytes() of device memory
+    int n = 0;              // shifts
+    VecBlock *xs = nullptr, *ps = nullptr;  // device arrays by shift
+    VecBlock hist;
+    MsHistEntry *hist_s = nullptr;
+};
+bool solver_loop_run(Prec pv, const LoopRun &q, const Launch &L);
+size_t solver_loop_slot_bytes();
+// the loop would read mirrored links of this set as such (loop.cu has the rule)
+bool loop_wants_mirrored(const LinkSet &ls, int vh);
+// Whether every backward link of ls (FP64 or FP32, 18 reals) equals, bit for
+// bit, the forward link of its own site (as MILC's backward links do), with
+// periodic wrap on the lattice of L.  d_flag: an int of device memory.
+bool links_mirrored(const LinkSet &ls, const Launch &L, int *d_flag);
+// a Dslash variant was chosen by the caller or the environment
+bool dslash_variant_forced();
 
 // elementwise helpers
 void vec_copy(Prec dst_p, VecBlock dst, Prec src_p, VecBlock src, const Launch &L);

@@ -153,8 +153,10 @@ public:
     // host time spent capturing and instantiating graphs so far
     double build_seconds() const { return build_sec_; }
 
+    // `res`: the phase as the resident loop takes it (loop.cu), with vectors
+    // in `pv`; nullptr when it has no such form
     template <typename Enq, typename Next>
-    void run(Enq enqueue, Next next, TimedLaunches &tl, int cap, int first_chunk = 8)
+    void run(Enq enqueue, Next next, TimedLaunches &tl, int cap, Prec pv, LoopRun *res, int first_chunk = 8)
     {
         Context &c = ctx();
         SolverState &S = *c.h_state;
@@ -162,6 +164,20 @@ public:
         S.skip_axpy = 0;
         S.err = c.d_err;
         S.counter = S.counter2 = 0;
+        if (res && graphs_enabled() && !tl.on && !c.halo.on) {
+            res->st = c.d_state;
+            res->slots = c.d_slots;
+            S.use_cond = 0;
+            S.iter_cap = S.iteration + (cap > 0 ? cap : 1);
+            S.err = nullptr;  // the loop reports a failed wait itself
+            upload_state();
+            if (solver_loop_run(pv, *res, c.launch())) {
+                download_state();
+                if (S.stop_at == INT_MAX) throw Error("solver: device loop ended without a stop");
+                return;
+            }
+            S.err = c.d_err;
+        }
         // NCCL calls are not captured: a solve over several GPUs runs in chunks
         if (graphs_enabled() && !tl.on && !(c.halo.on && c.halo.nranks > 1)) {
             if (!exec_) {
@@ -365,6 +381,12 @@ int cg_reference(Prec P, const LinkSet &ls, SolveArgs &A)
             S.size_r = res->size_r;
             S.size_relr = res->size_relr;
             double size_prev = res->size_r > 0 ? res->size_r : 1.0;
+            LoopRun lr;
+            lr.mode = kLoopCg;
+            lr.links = &ls;
+            lr.parity = parity;
+            lr.p = cg_p; lr.tmp = tmp; lr.ttt = ttt; lr.r = resid; lr.x = t_dest;
+            lr.m4 = -msq_x4;
             loop.run(
                 [&](int k) {
                     tl.run(0, k, [&] { dslash_gated(P, L, tmp, cg_p, ls, otherparity, c.d_state, k); });
@@ -380,7 +402,7 @@ int cg_reference(Prec P, const LinkSet &ls, SolveArgs &A)
                     size_prev = S.size_r;
                     return n;
                 },
-                tl, niter - (iteration % niter) + 1);
+                tl, niter - (iteration % niter) + 1, P, relres ? nullptr : &lr);
             if (S.error) breakdown("asqtad_invert", S.error, S.iteration);
             iteration = S.iteration;
             rsq = S.rsq;
@@ -531,6 +553,13 @@ MixedResult mixed_pass(Prec ps, const LinkSet &ls64, const LinkSet &lss, const L
     lap(out.t_setup);
     for (;;) {
         double size_prev = S.rsq;
+        LoopRun lr;
+        lr.mode = kLoopMx;
+        lr.links = ls_cur;
+        lr.parity = parity;
+        lr.p = pv; lr.tmp = tmps; lr.ttt = ttts; lr.r = rs; lr.x = xs;
+        lr.m4 = -m4;
+        lr.delta2 = delta2;
         loop.run(
             [&](int k) {
                 tl.run(0, k, [&] { dslash_gated(ps, L, tmps, pv, *ls_cur, other, c.d_state, k); });
@@ -546,7 +575,7 @@ MixedResult mixed_pass(Prec ps, const LinkSet &ls64, const LinkSet &lss, const L
                 size_prev = S.rsq;
                 return n;
             },
-            tl, max_cg - S.iteration + 1);
+            tl, max_cg - S.iteration + 1, ps, &lr);
         if (S.error) breakdown("asqtad_invert (mixed precision)", S.error, S.iteration);
         lap(out.t_loop);
         out.iterations = S.iteration;
@@ -837,6 +866,15 @@ MsPass ms_pass(Prec p, Prec xp, const LinkSet &ls, VecBlock src, std::vector<Vec
     for (;;) {
         S.ms_ru = 0;
         const double t0 = c.verbose ? wall_seconds() : 0.0;
+        LoopRun lr;
+        lr.mode = df ? kLoopMsDefer : kLoopMs;
+        lr.links = &ls;
+        lr.parity = parity;
+        lr.p = pm[j_low]; lr.tmp = tmp; lr.ttt = ttt; lr.r = resid;
+        lr.m4 = m4;
+        lr.n = n;
+        lr.xs = d_x; lr.ps = d_p;
+        if (df) { lr.hist = df->hist(); lr.hist_s = df->hist_scalars(); }
         loop.run(
             [&](int k) {
                 tl.run(0, k, [&] { dslash_gated(p, L, tmp, pm[j_low], ls, other, c.d_state, k); });
@@ -852,7 +890,7 @@ MsPass ms_pass(Prec p, Prec xp, const LinkSet &ls, VecBlock src, std::vector<Vec
                 size_prev = S.rsq;
                 return m;
             },
-            tl, max_cg + 1);
+            tl, max_cg + 1, p, df || xp == p ? &lr : nullptr);
         if (S.error) breakdown("asqtad_invert_multi", S.error, S.iteration);
         const bool seg_full = S.ms_seg_full != 0;
         const double t1 = c.verbose ? wall_seconds() : 0.0;

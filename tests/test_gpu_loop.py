@@ -1,0 +1,94 @@
+"""GPU: the resident solver loop (one cooperative launch per solver phase)
+against the launch-per-kernel loop (QPHIX_B200_LOOP=0) of the same solvers.
+
+A fixed, small number of iterations is compared, so that the results differ
+by the rounding of differently ordered sums only: after n iterations of a
+well-conditioned system (m = 0.3, condition number about 100) they agree to a
+few hundred units of the storage's rounding (FP64 1e-12, FP32 1e-4 of the
+largest component; 16-bit storages round both alike and add 2^-15 per
+vector store, 1e-3).  The lattices are the smallest, ragged ones, and ones on
+either side of the loop's rules: groups of 4..32 sites, eight or four parts a
+site, links read once per site (mirrored).
+"""
+import numpy as np
+import pytest
+
+from conftest import fields, rel_err, synthetic
+
+pytestmark = pytest.mark.gpu
+
+# sites per parity 128, 256, 768, 2304 (ragged), 20736 (four parts in FP32),
+# 32768 (mirrored FP32 and FP64; four parts in FP64)
+DIMS = [(4, 4, 4, 4), (4, 8, 4, 4), (8, 4, 4, 12), (12, 8, 4, 12), (12, 12, 12, 24), (16, 16, 16, 16)]
+MODES = {"double": 1e-12, "F": 1e-4, "single": 1e-4, "r12": 1e-4, "half-links": 1e-4, "half": 1e-3}
+
+
+def _solve(lib, mode, links, src, parity, n, masses):
+    prec = "F" if mode == "F" else "D"
+    lib.set_inner_precision({"F": "double", "r12": "single"}.get(mode, mode))
+    lib.set_link_compression(mode == "r12")
+    try:
+        L = lib.create_L(prec, links)
+        b = lib.create_V(prec, src, parity)
+        xs = [lib.create_V(prec, np.zeros_like(src), parity) for _ in masses]
+        if len(masses) == 1:
+            it, info, _ = lib.invert(prec, L, xs[0], b, masses[0], parity=parity, max_iter=n, nrestart=1, resid=1e-30)
+        else:
+            it, info, _ = lib.invert_multi(prec, L, xs, b, masses, parity=parity, max_iter=n, nrestart=1, resid=1e-30)
+        assert info.status == 0, lib.last_error()
+        out = [lib.extract_V(prec, x, parity) for x in xs]
+        for h in xs + [b]:
+            lib.destroy_V(prec, h)
+        lib.destroy_L(prec, L)
+        return it, out
+    finally:
+        lib.set_inner_precision("double")
+        lib.set_link_compression(False)
+
+
+def _both(lib, monkeypatch, *args):
+    monkeypatch.setenv("QPHIX_B200_LOOP", "0")
+    ref = _solve(lib, *args)
+    monkeypatch.delenv("QPHIX_B200_LOOP")
+    return _solve(lib, *args), ref
+
+
+@pytest.mark.parametrize("dims", DIMS, ids=lambda d: "x".join(map(str, d)))
+@pytest.mark.parametrize("mode", list(MODES))
+def test_cg_iterations(gpu, monkeypatch, dims, mode):
+    lib = gpu.use(dims)
+    parity = "odd" if dims[3] == 12 else "even"
+    src = synthetic.gaussian_source(dims, seed=5, parity=parity)
+    (it, x), (it0, x0) = _both(lib, monkeypatch, mode, fields(dims), src, parity, 12, [0.3])
+    assert it == it0
+    assert rel_err(x[0], x0[0]) < MODES[mode]
+
+
+@pytest.mark.parametrize("dims", [(4, 4, 4, 4), (12, 8, 4, 12), (12, 12, 12, 24)], ids=lambda d: "x".join(map(str, d)))
+@pytest.mark.parametrize("mode", ["double", "F", "r12"])
+def test_multishift_iterations(gpu, monkeypatch, dims, mode):
+    """kLoopMs (FP64, FP32) and kLoopMsDefer (mixed)."""
+    lib = gpu.use(dims)
+    src = synthetic.gaussian_source(dims, seed=6, parity="even")
+    masses = [0.5, 0.3, 0.4]
+    (it, x), (it0, x0) = _both(lib, monkeypatch, mode, fields(dims), src, "even", 10, masses)
+    assert it == it0
+    for a, b in zip(x, x0):
+        assert rel_err(a, b) < MODES[mode]
+
+
+@pytest.mark.parametrize("mode", ["double", "F", "single"])
+def test_backward_links_that_are_not_shifted_forward_links(gpu, monkeypatch, mode):
+    """One backward link changed: the loop must read the caller's backward
+    links, not the forward ones of their sites.  (The operator is then not
+    Hermitian; the iterations are compared, not a solution.)"""
+    dims = (16, 16, 16, 16)
+    lib = gpu.use(dims)
+    src = synthetic.gaussian_source(dims, seed=7, parity="even")
+    links = dict(fields(dims))
+    changed = dict(links, fatback=links["fatback"].copy())
+    changed["fatback"][72 * 1234:72 * 1234 + 18] *= 1.5
+    (_, x), (_, x0) = _both(lib, monkeypatch, mode, changed, src, "even", 6, [0.3])
+    assert rel_err(x[0], x0[0]) < MODES[mode]
+    _, y = _solve(lib, mode, links, src, "even", 6, [0.3])
+    assert rel_err(y[0], x0[0]) > 30 * MODES["single" if mode != "double" else "double"]
