@@ -23,9 +23,16 @@
 // reference, one call updates the links of one checkerboard: the objects'
 // parity, EVENODD meaning EVEN (qphix_f3.cpp:178-179, 347-348).
 //
-// One thread owns one link (site of the parity, direction mu) and walks the
-// 48 staple paths of a constant table; the links it gathers come from
-// L1/L2 (every link is read by ~200 threads).  FP64 for D3, FP32 for F3.
+// One thread owns one link (site of the parity, direction mu).  The 48
+// staples are not walked one by one: with A = the step (nu, s) from x + mu,
+// C = the step (-rho, -r) into x and W the steps between, the plaquettes,
+// the rectangles that end with a rho step and all parallelograms are
+//   sum_{rho r} ( sum_{nu s} A W ) C,
+// so the products that end in the same step are summed before the last
+// multiplication (gf_program): 134 products of 3x3 matrices and 182 link
+// loads per link instead of 181 and 229.  The links come from L1/L2 (every
+// link is read by ~150 threads).  FP64 for D3, FP32 for F3.
+#include <algorithm>
 #include <cstring>
 #include <type_traits>
 #include <vector>
@@ -37,194 +44,279 @@ namespace qb {
 
 namespace {
 
-// staple paths of a forward link mu: steps 2*axis (forward) or 2*axis+1
-// (backward) from x + mu back to x; type 0 plaquette, 1 rectangle, 2
-// parallelogram
-struct GfPath {
-    unsigned char n, type, s[5];
+// One entry of the evaluation of a link's staple sum: a link U (its adjoint
+// when the path passes it backwards) and what is done with it.
+//   kStart  M = U
+//   kMul    M = M U
+//   kMix    M = c1 M + c0 U
+//   kFold   S = S + X U; X = 0
+// and, when `add` is 1 + t, then X = X + c_t M (c_0 plaquette, c_1
+// rectangle, c_2 parallelogram coefficient), when it is 4, X = X + M.  The
+// link's site is x plus a displacement of -2..2 along each axis, kept in the
+// entry, so that a thread only adds up the block indices of its own wrapped
+// coordinates.
+enum GfOp : unsigned { kStart = 0, kMul = 1, kMix = 2, kFold = 3 };
+// bits: 0-1 op, 2-3 axis of U, 4 adjoint, 5-7 add, 8 parity of the
+// displacement, 9 + 3a .. 11 + 3a displacement along a plus 2
+struct GfEntry {
+    static unsigned make(GfOp op, int axis, bool adj, int add, const int disp[4])
+    {
+        unsigned e = (unsigned)op | (unsigned)axis << 2 | (unsigned)adj << 4 | (unsigned)add << 5;
+        e |= (unsigned)((disp[0] + disp[1] + disp[2] + disp[3]) & 1) << 8;
+        for (int a = 0; a < 4; ++a) e |= (unsigned)(disp[a] + 2) << (9 + 3 * a);
+        return e;
+    }
 };
-constexpr int kGfPaths = 48;
-__constant__ GfPath c_gf_paths[4][kGfPaths];
+constexpr int kGfProgram = 184;  // entries of the longest program
+// programs by which coefficients are non-zero (bit t: c_t) and direction
+__constant__ unsigned c_gf_program[8][4][kGfProgram];
+__constant__ int c_gf_length[8][4];
 
-std::vector<GfPath> staple_table(int mu)
+// The program of direction mu; terms with a zero coefficient are left out.
+std::vector<unsigned> gf_program(int mask, int mu)
 {
-    std::vector<GfPath> out;
-    int others[3], k = 0;
-    for (int d = 0; d < 4; ++d)
-        if (d != mu) others[k++] = d;
-    auto st = [](int axis, int sign) { return (unsigned char)(2 * axis + (sign < 0 ? 1 : 0)); };
-    for (int i = 0; i < 3; ++i)
-        for (int s : {1, -1}) {
-            const int nu = others[i];
-            out.push_back(GfPath{3, 0, {st(nu, s), st(mu, -1), st(nu, -s), 0, 0}});
-        }
-    for (int i = 0; i < 3; ++i)
-        for (int s : {1, -1}) {
-            const int nu = others[i];
-            out.push_back(GfPath{5, 1, {st(mu, 1), st(nu, s), st(mu, -1), st(mu, -1), st(nu, -s)}});
-            out.push_back(GfPath{5, 1, {st(nu, s), st(mu, -1), st(mu, -1), st(nu, -s), st(mu, 1)}});
-            out.push_back(GfPath{5, 1, {st(nu, s), st(nu, s), st(mu, -1), st(nu, -s), st(nu, -s)}});
-        }
-    for (int i = 0; i < 3; ++i)
-        for (int i2 = 0; i2 < 3; ++i2) {
-            if (i2 == i) continue;
-            for (int s : {1, -1})
-                for (int r : {1, -1}) {
-                    const int nu = others[i], rho = others[i2];
-                    out.push_back(GfPath{5, 2, {st(nu, s), st(rho, r), st(mu, -1), st(nu, -s), st(rho, -r)}});
+    std::vector<unsigned> p;
+    const bool c0 = mask & 1, c1 = mask & 2, c2 = mask & 4;
+    int pos[4] = {0, 0, 0, 0};
+    // one step of a path from the current position (kStart and kMix: from x + mu)
+    auto add = [&](GfOp op, int axis, int sign, int coef = 0) {
+        if (op == kStart || op == kMix)
+            for (int d = 0; d < 4; ++d) pos[d] = d == mu;
+        if (sign < 0) --pos[axis];
+        p.push_back(GfEntry::make(op, axis, sign < 0, coef, pos));
+        if (sign > 0) ++pos[axis];
+    };
+    if (!mask) return p;
+    for (int rho = 0; rho < 4; ++rho) {
+        if (rho == mu) continue;
+        for (int r : {1, -1}) {
+            if (c2)
+                for (int nu = 0; nu < 4; ++nu) {
+                    if (nu == mu || nu == rho) continue;
+                    for (int s : {1, -1}) {  // parallelogram [nu s, rho r, -mu, -nu s, -rho r]
+                        add(kStart, nu, s);
+                        add(kMul, rho, r);
+                        add(kMul, mu, -1);
+                        add(kMul, nu, -s, 3);
+                    }
                 }
+            if (c1) {
+                // rectangle [rho r, rho r, -mu, -rho r, -rho r]
+                add(kStart, rho, r);
+                add(kMul, rho, r);
+                add(kMul, mu, -1);
+                add(kMul, rho, -r, 2);
+                // rectangle [mu, rho r, -mu, -mu, -rho r] and the plaquette
+                // [rho r, -mu, -rho r], whose last two steps are the same
+                add(kStart, mu, 1);
+                add(kMul, rho, r);
+                add(kMul, mu, -1);
+                if (c0) {
+                    add(kMix, rho, r);
+                    add(kMul, mu, -1, 4);  // (the weights are in M)
+                } else {
+                    add(kMul, mu, -1, 2);
+                }
+            } else if (c0) {
+                add(kStart, rho, r);
+                add(kMul, mu, -1, 1);
+            }
+            add(kFold, rho, -r);
         }
-    return out;
+    }
+    if (c1) {  // rectangles [nu s, -mu, -mu, -nu s, mu]
+        for (int nu = 0; nu < 4; ++nu) {
+            if (nu == mu) continue;
+            for (int s : {1, -1}) {
+                add(kStart, nu, s);
+                add(kMul, mu, -1);
+                add(kMul, mu, -1);
+                add(kMul, nu, -s, 2);
+            }
+        }
+        add(kFold, mu, 1);
+    }
+    return p;
 }
 
-// 3x3 complex products on row-major reals (u[6 r + 2 c] + i u[6 r + 2 c + 1])
-template <typename R>
-__device__ __forceinline__ void mm(const R a[18], const R b[18], R c[18], bool adj_b)
+// One row of a product of 3x3 complex matrices (row-major reals u[6 r + 2 c] +
+// i u[6 r + 2 c + 1]): t = (a_0, a_1, a_2) b or b^dag, as chains of fused
+// multiply-adds: two per pair of real products, where re += ar * br - ai * bi
+// compiles to three instructions.
+template <bool ADJ, typename R>
+__device__ __forceinline__ void mm_row(const R a[6], const R b[18], R t[6])
 {
 #pragma unroll
-    for (int r = 0; r < 3; ++r)
+    for (int k = 0; k < 3; ++k) {
+        R re = R(0), im = R(0);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            R re = 0, im = 0;
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                const R ar = a[6 * r + 2 * j], ai = a[6 * r + 2 * j + 1];
-                // b_jk, or conj(b_kj) for b^dag
-                const R br = adj_b ? b[6 * k + 2 * j] : b[6 * j + 2 * k];
-                const R bi = adj_b ? -b[6 * k + 2 * j + 1] : b[6 * j + 2 * k + 1];
-                re += ar * br - ai * bi;
-                im += ar * bi + ai * br;
-            }
-            c[6 * r + 2 * k] = re;
-            c[6 * r + 2 * k + 1] = im;
+        for (int j = 0; j < 3; ++j) {
+            const R ar = a[2 * j], ai = a[2 * j + 1];
+            const R br = ADJ ? b[6 * k + 2 * j] : b[6 * j + 2 * k];
+            const R bi = ADJ ? b[6 * k + 2 * j + 1] : b[6 * j + 2 * k + 1];  // (conjugated below)
+            re = j == 0 ? ar * br : fma_(ar, br, re);
+            im = j == 0 ? ai * br : fma_(ai, br, im);
+            re = ADJ ? fma_(ai, bi, re) : fma_(-ai, bi, re);
+            im = ADJ ? fma_(-ar, bi, im) : fma_(ar, bi, im);
         }
+        t[2 * k] = re;
+        t[2 * k + 1] = im;
+    }
+}
+
+// a = a b or a b^dag (a row of the product needs only that row of a)
+template <bool ADJ, typename R>
+__device__ __forceinline__ void mm_inplace(R a[18], const R b[18])
+{
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        R t[6];
+        mm_row<ADJ>(a + 6 * r, b, t);
+#pragma unroll
+        for (int i = 0; i < 6; ++i) a[6 * r + i] = t[i];
+    }
 }
 
 template <typename R>
 struct GaugeView {
     const cx_t<R> *b[2];
     Geom g;
-    // link of direction d at full coordinates y (already wrapped)
-    __device__ __forceinline__ void load(const int y[4], int d, R u[18]) const
-    {
-        const int cb = (y[0] + y[1] + y[2] + y[3]) & 1;
-        const int j = ((y[3] * g.nz + y[2]) * g.ny + y[1]) * g.nxh + (y[0] >> 1);
-        const cx_t<R> *p = b[cb] + (size_t)d * 9 * g.vh + j;
-#pragma unroll
-        for (int e = 0; e < 9; ++e) {
-            const cx_t<R> z = __ldg(p + (size_t)e * g.vh);
-            u[2 * e] = z.x;
-            u[2 * e + 1] = z.y;
-        }
-    }
 };
 
-// M <- M U or M U^dag, one row at a time (row r of the product needs only
-// row r of M), with mm's arithmetic order
+// One thread per link (direction-major: a warp's threads share the program
+// and gather consecutive sites).  What bounds it at 12 warps per SM is the
+// instruction issue and the latency of the gathers, so
+//  * the next entry's link is loaded before the product with the current one
+//    (two links, M and X in registers; the loop is unrolled by two so that no
+//    link is copied);
+//  * the block indices of the wrapped coordinates x - 2 .. x + 2 along each
+//    axis are computed once into shared memory;
+//  * adjoints are taken in the product, by a branch the whole warp takes;
+//  * the staple sum S, used seven times per link, is in shared memory.
+constexpr int kGfThreads = 128;
+template <typename R> struct GfMinBlocks { static constexpr int value = 5; };
+template <> struct GfMinBlocks<double> { static constexpr int value = 3; };
+
 template <typename R>
-__device__ __forceinline__ void mm_inplace(R a[18], const R b[18], bool adj_b)
+struct GfShared {
+    R acc[18][kGfThreads];
+    int idx[4][5][kGfThreads];  // by axis and displacement + 2
+};
+
+template <typename R>
+__device__ __forceinline__ void gf_load(const GaugeView<R> &U, const GfShared<R> &sh, int cb, unsigned e, R u[18])
 {
+    const int tid = threadIdx.x, vh = U.g.vh;
+    const int j = sh.idx[0][(e >> 9) & 7][tid] + sh.idx[1][(e >> 12) & 7][tid] + sh.idx[2][(e >> 15) & 7][tid] +
+                  sh.idx[3][(e >> 18) & 7][tid];
+    const cx_t<R> *p = U.b[(cb ^ (e >> 8)) & 1] + (size_t)((e >> 2) & 3) * 9 * vh + j;
 #pragma unroll
-    for (int r = 0; r < 3; ++r) {
-        R t[6];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            R re = 0, im = 0;
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                const R ar = a[6 * r + 2 * j], ai = a[6 * r + 2 * j + 1];
-                const R br = adj_b ? b[6 * k + 2 * j] : b[6 * j + 2 * k];
-                const R bi = adj_b ? -b[6 * k + 2 * j + 1] : b[6 * j + 2 * k + 1];
-                re += ar * br - ai * bi;
-                im += ar * bi + ai * br;
-            }
-            t[2 * k] = re;
-            t[2 * k + 1] = im;
-        }
-#pragma unroll
-        for (int i = 0; i < 6; ++i) a[6 * r + i] = t[i];
+    for (int k = 0; k < 9; ++k) {
+        const cx_t<R> z = __ldg(p + (size_t)k * vh);
+        u[2 * k] = z.x;
+        u[2 * k + 1] = z.y;
     }
 }
 
-// One thread per link (direction-major: a warp's threads share the path
-// table entry and gather consecutive sites).  In FP64 the path product is
-// formed in place, one row at a time, under a register cap of four blocks per
-// SM: 15.6 ms against 16.2 ms per 32^3x64 checkerboard.  In FP32 both were
-// slower (9.7 ms with the cap, 10.6 ms in place without it, against 9.3 ms),
-// so FP32 keeps the product in a third matrix.  Moving the staple sum to
-// shared memory and interleaving the four directions of a site over adjacent
-// threads was slower in both (17.4 / 11.8 ms).
-constexpr int kGfThreads = 128;
-template <typename R> struct GfMinBlocks { static constexpr int value = 1; };
-template <> struct GfMinBlocks<double> { static constexpr int value = 4; };
+template <bool ADJ, typename R>
+__device__ __forceinline__ void gf_apply(GfShared<R> &sh, unsigned op, const R u[18], R M[18], R X[18], R c0, R c1)
+{
+    if (op == kMul) {
+        mm_inplace<ADJ>(M, u);
+    } else if (op == kFold) {
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            R t[6];
+            mm_row<ADJ>(X + 6 * r, u, t);
+#pragma unroll
+            for (int k = 0; k < 6; ++k) {
+                sh.acc[6 * r + k][threadIdx.x] += t[k];
+                X[6 * r + k] = R(0);
+            }
+        }
+    } else {
+        const bool mix = op == kMix;
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const R x = ADJ ? u[6 * k + 2 * r] : u[6 * r + 2 * k];
+                const R y = ADJ ? -u[6 * k + 2 * r + 1] : u[6 * r + 2 * k + 1];
+                M[6 * r + 2 * k] = mix ? fma_(c1, M[6 * r + 2 * k], c0 * x) : x;
+                M[6 * r + 2 * k + 1] = mix ? fma_(c1, M[6 * r + 2 * k + 1], c0 * y) : y;
+            }
+    }
+}
 
 template <typename R>
 __global__ void __launch_bounds__(kGfThreads, GfMinBlocks<R>::value)
-k_gauge_force(GaugeView<R> U, cx_t<R> *mom, int cb, R eps, R c0, R c1, R c2)
+k_gauge_force(GaugeView<R> U, cx_t<R> *mom, int cb, R eps, R c0, R c1, R c2, int mask)
 {
+    __shared__ GfShared<R> sh;
     const Geom &g = U.g;
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    const int idx = blockIdx.x * blockDim.x + threadIdx.x, tid = threadIdx.x;
     if (idx >= 4 * g.vh) return;
     const int mu = idx / g.vh, j = idx - mu * g.vh;
-    const SiteCoords s = decode(g, cb, j);
-    const int x0[4] = {2 * s.xh + s.xodd, s.y, s.z, s.t};
-    const int L[4] = {g.nx, g.ny, g.nz, g.nt};
-    const R coef[3] = {c0, c1, c2};
-    R acc[18];
+    {
+        const SiteCoords s = decode(g, cb, j);
+        const int x = 2 * s.xh + s.xodd;
 #pragma unroll
-    for (int i = 0; i < 18; ++i) acc[i] = R(0);
-#pragma unroll 1
-    for (int p = 0; p < kGfPaths; ++p) {
-        const GfPath P = c_gf_paths[mu][p];
-        const R c = coef[P.type];
-        if (c == R(0)) continue;
-        int y[4] = {x0[0], x0[1], x0[2], x0[3]};
-        y[mu] = y[mu] + 1 == L[mu] ? 0 : y[mu] + 1;
-        R M[18], Lk[18];
-#pragma unroll 1
-        for (int k = 0; k < P.n; ++k) {
-            const int a = P.s[k] >> 1;
-            const bool back = P.s[k] & 1;
-            if (back) y[a] = y[a] == 0 ? L[a] - 1 : y[a] - 1;
-            U.load(y, a, Lk);
-            if (!back) y[a] = y[a] + 1 == L[a] ? 0 : y[a] + 1;
-            if (k == 0) {
-                if (back) {
-#pragma unroll
-                    for (int r = 0; r < 3; ++r)
-#pragma unroll
-                        for (int q = 0; q < 3; ++q) {
-                            M[6 * r + 2 * q] = Lk[6 * q + 2 * r];
-                            M[6 * r + 2 * q + 1] = -Lk[6 * q + 2 * r + 1];
-                        }
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 18; ++i) M[i] = Lk[i];
-                }
-            } else if constexpr (std::is_same<R, double>::value) {
-                mm_inplace(M, Lk, back);
-            } else {
-                R T[18];
-                mm(M, Lk, T, back);
-#pragma unroll
-                for (int i = 0; i < 18; ++i) M[i] = T[i];
-            }
+        for (int o = -2; o <= 2; ++o) {  // (every extent is at least 4)
+            sh.idx[0][o + 2][tid] = wrap(x + o, g.nx) >> 1;
+            sh.idx[1][o + 2][tid] = wrap(s.y + o, g.ny) * g.sy;
+            sh.idx[2][o + 2][tid] = wrap(s.z + o, g.nz) * g.sz;
+            sh.idx[3][o + 2][tid] = wrap(s.t + o, g.nt) * g.st;
         }
-#pragma unroll
-        for (int i = 0; i < 18; ++i) acc[i] += c * M[i];
     }
-    R Um[18], W[18];
-    U.load(x0, mu, Um);
-    mm(Um, acc, W, false);
+    R M[18], X[18], ua[18], ub[18];
+#pragma unroll
+    for (int i = 0; i < 18; ++i) {
+        X[i] = M[i] = R(0);
+        sh.acc[i][tid] = R(0);
+    }
+    const unsigned *prog = c_gf_program[mask][mu];
+    const int n = c_gf_length[mask][mu];
+    auto apply = [&](unsigned e, const R u[18]) {
+        if (e & 16u) gf_apply<true>(sh, e & 3u, u, M, X, c0, c1);
+        else gf_apply<false>(sh, e & 3u, u, M, X, c0, c1);
+        const unsigned add = (e >> 5) & 7u;
+        if (add) {
+            const R c = add == 1 ? c0 : add == 2 ? c1 : add == 3 ? c2 : R(1);
+#pragma unroll
+            for (int k = 0; k < 18; ++k) X[k] = fma_(c, M[k], X[k]);
+        }
+    };
+    if (n) gf_load(U, sh, cb, prog[0], ua);
+#pragma unroll 1
+    for (int i = 0; i < n; i += 2) {
+        if (i + 1 < n) gf_load(U, sh, cb, prog[i + 1], ub);
+        apply(prog[i], ua);
+        if (i + 1 < n) {
+            if (i + 2 < n) gf_load(U, sh, cb, prog[i + 2], ua);
+            apply(prog[i + 1], ub);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 18; ++i) X[i] = sh.acc[i][tid];
+    {
+        const cx_t<R> *p = U.b[cb] + (size_t)mu * 9 * g.vh + j;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            const cx_t<R> z = __ldg(p + (size_t)k * g.vh);
+            M[2 * k] = z.x;
+            M[2 * k + 1] = z.y;
+        }
+    }
+    mm_inplace<false>(M, X);  // W = U S
     // TA(W) = (W - W^dag)/2 - tr(W - W^dag)/6
-    const R tr = (W[1] + W[9] + W[17]) * (R(1) / R(3));  // imaginary part of tr(W - W^dag)/2 / 3
+    const R tr = (M[1] + M[9] + M[17]) * (R(1) / R(3));  // imaginary part of tr(W - W^dag)/2 / 3
     cx_t<R> *m = mom + (size_t)mu * 9 * g.vh + j;
 #pragma unroll
     for (int r = 0; r < 3; ++r)
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
-            R fr = R(0.5) * (W[6 * r + 2 * q] - W[6 * q + 2 * r]);
-            R fi = R(0.5) * (W[6 * r + 2 * q + 1] + W[6 * q + 2 * r + 1]);
+            R fr = R(0.5) * (M[6 * r + 2 * q] - M[6 * q + 2 * r]);
+            R fi = R(0.5) * (M[6 * r + 2 * q + 1] + M[6 * q + 2 * r + 1]);
             if (r == q) fi -= tr;
             cx_t<R> z = m[(size_t)(3 * r + q) * g.vh];
             z.x += eps * fr;
@@ -450,26 +542,29 @@ void upload_table()
     int dev = 0;
     QB_CUDA(cudaGetDevice(&dev));
     if (dev >= 0 && dev < 64 && g_table_ready[dev]) return;
-    GfPath t[4][kGfPaths];
-    for (int mu = 0; mu < 4; ++mu) {
-        const std::vector<GfPath> p = staple_table(mu);
-        if ((int)p.size() != kGfPaths) throw Error("gauge force: staple table has the wrong size");
-        for (int i = 0; i < kGfPaths; ++i) t[mu][i] = p[i];
-    }
-    QB_CUDA(cudaMemcpyToSymbol(c_gf_paths, t, sizeof(t)));
+    static unsigned prog[8][4][kGfProgram];
+    int len[8][4];
+    for (int mask = 0; mask < 8; ++mask)
+        for (int mu = 0; mu < 4; ++mu) {
+            const std::vector<unsigned> p = gf_program(mask, mu);
+            if ((int)p.size() > kGfProgram) throw Error("gauge force: program too long");
+            len[mask][mu] = (int)p.size();
+            std::copy(p.begin(), p.end(), prog[mask][mu]);
+        }
+    QB_CUDA(cudaMemcpyToSymbol(c_gf_program, prog, sizeof(prog)));
+    QB_CUDA(cudaMemcpyToSymbol(c_gf_length, len, sizeof(len)));
     if (dev >= 0 && dev < 64) g_table_ready[dev] = true;
 }
 
-// flops of one link's force: (steps - 1) 3x3 complex products per path
-// (198 flops each), its weighted sum (36), U times the sum (198), TA and the
-// update (54)
+// flops of one link's force, loop by loop: 2 (plaquette) or 4 (six-link
+// loops) 3x3 complex products per staple (198 flops each), its weighted sum
+// (36), U times the sum (198), TA and the update (54)
 double flops_per_link(const QPHIX_gauge_coeffs_t &co)
 {
-    const double c[3] = {co.plaquette, co.rectangle, co.parallelogram};
-    const std::vector<GfPath> p = staple_table(0);
     double f = 198 + 54;
-    for (const auto &q : p)
-        if (c[q.type] != 0.0) f += 198.0 * (q.n - 1) + 36;
+    if (co.plaquette != 0.0) f += 6 * (198.0 * 2 + 36);
+    if (co.rectangle != 0.0) f += 18 * (198.0 * 4 + 36);
+    if (co.parallelogram != 0.0) f += 24 * (198.0 * 4 + 36);
     return f;
 }
 
@@ -493,9 +588,10 @@ void gauge_force(QPHIX_info_t *info, typename GfApi<R>::G *G, typename GfApi<R>:
         U.g = c.g;
         QB_CUDA(cudaEventRecord(c.ev_solve[0], c.stream));
         const int grid = (4 * c.g.vh + kGfThreads - 1) / kGfThreads;
-        k_gauge_force<R><<<grid, kGfThreads, 0, c.stream>>>(U, static_cast<cx_t<R> *>(F->blk[cb]), cb, eps,
-                                                     (R)coeffs->plaquette, (R)coeffs->rectangle,
-                                                     (R)coeffs->parallelogram);
+        const R co[3] = {(R)coeffs->plaquette, (R)coeffs->rectangle, (R)coeffs->parallelogram};
+        const int mask = (co[0] != R(0) ? 1 : 0) | (co[1] != R(0) ? 2 : 0) | (co[2] != R(0) ? 4 : 0);
+        k_gauge_force<R><<<grid, kGfThreads, 0, c.stream>>>(U, static_cast<cx_t<R> *>(F->blk[cb]), cb, eps, co[0],
+                                                            co[1], co[2], mask);
         QB_CUDA(cudaGetLastError());
         QB_CUDA(cudaEventRecord(c.ev_solve[1], c.stream));
         sync_check();

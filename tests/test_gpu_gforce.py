@@ -126,3 +126,25 @@ def test_gauge_force_rejects_null_arguments(gpu):
         assert "NULL" in lib.last_error()
     finally:
         lib.destroy_G("D", g)
+
+
+@pytest.mark.parametrize("dims", [(4, 4, 4, 4), (12, 4, 8, 4)])
+@pytest.mark.parametrize("which", range(1, 8))
+def test_gauge_force_of_every_subset_of_loops(gpu, dims, which):
+    """Each subset of non-zero coefficients has its own program of products
+    (bit 0 plaquette, 1 rectangle, 2 parallelogram); on extents of 4 every
+    displacement of two wraps.  FP64 sums of 48 products of at most five
+    matrices: 1e-12 of the largest momentum."""
+    lib = gpu.use(dims)
+    lat, U, A, Uraw, Araw = _fields(dims)
+    co = {k: v if which >> i & 1 else 0.0
+          for i, (k, v) in enumerate((("plaquette", 0.7), ("rectangle", -0.2), ("parallelogram", 0.3)))}
+    for parity in ("even", "odd"):
+        g, f = lib.create_G("D", Uraw, parity), lib.create_F("D", Araw, parity)
+        assert lib.gauge_force("D", g, f, co, 0.5).status == 0, lib.last_error()
+        got = _lex(dims, lib.extract_F("D", f, parity))
+        mask = G.parity_mask(dims, parity)
+        want = G.momentum_update(U, A, co, 0.5, mask) * mask[..., None, None, None]
+        assert np.abs(got - want).max() < 1e-12 * np.abs(want).max()
+        lib.destroy_F("D", f)
+        lib.destroy_G("D", g)
