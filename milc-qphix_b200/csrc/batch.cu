@@ -222,6 +222,30 @@ __device__ __forceinline__ void b_masks(BState *st)
     st->flag_mask = f;
 }
 
+// Systems of a segment take their reliable updates together: when one is
+// due, so is every active one whose |r|^2 has halved since its last update.
+// An update of a single system streams the FP64 links of the whole lattice
+// and runs every warp with a few of its lanes, so it costs nearly what the
+// update of the whole segment does.
+constexpr double kBJoin = 0.5;
+__device__ __forceinline__ void b_flag_segments(const BTable *tab, BState *st)
+{
+    unsigned long long f = st->flag_mask;
+    for (int s = 0; s < tab->nseg; ++s) {
+        const int k0 = tab->seg[s].sys0, k1 = k0 + tab->seg[s].nrhs;
+        const unsigned long long m = (~0ull >> (64 - (k1 - k0))) << k0;
+        if (!(f & m) || (f & m) == m) continue;
+        for (int k = k0; k < k1; ++k) {
+            BSys &y = st->sys[k];
+            if (y.active && !y.flag && y.rsq < kBJoin * y.rsq_ru) {
+                y.flag = 1;
+                f |= 1ull << k;
+            }
+        }
+    }
+    st->flag_mask = f;
+}
+
 // ------------------------------------------------- multi-RHS vector loads --
 // 32-byte loads and stores (sm_100): four right-hand sides of one colour
 // component in one instruction, so the four threads of a site move a whole
@@ -743,6 +767,7 @@ __global__ void __launch_bounds__(kBlock) k_bvec(const BTable *tab, BState *st, 
                 },
                 [&] {
                     b_masks(st);
+                    if (st->flag_mask) b_flag_segments(tab, st);
                     st->any_flag = st->flag_mask != 0;
                     st->iteration += 1;
                     if (st->use_cond) cudaGraphSetConditional(st->cond_ru, st->any_flag ? 1u : 0u);
