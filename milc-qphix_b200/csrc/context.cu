@@ -36,15 +36,22 @@ void dev_free(void *p)
 
 namespace {
 
-constexpr size_t kStageBytes = 8u << 20;      // one pinned slot
-constexpr size_t kStageMinBytes = 16u << 20;  // smaller copies go in one call
+// One pinned slot, and the smallest copy that goes through the slots.  The
+// first slot's transfer and the last slot's host copy overlap nothing, so small
+// slots shorten both ends; with 1 MB the copies' own cost shows.  ms for
+// 191 MB device -> host / 32 MB device -> host / 1.5 GB host -> device, with
+// 8 workers and 8 MB slots 6.2 / 1.9 / 41, 8 and 2 MB 5.4 / 1.2 / 36, 12 and
+// 2 MB 4.9 / 1.2 / 35, 16 and 1 MB 4.8 / 1.3 / 43 (16 host cores).
+constexpr size_t kStageBytes = 2u << 20;
+constexpr size_t kStageMinBytes = 4u << 20;
+constexpr unsigned kStageWorkers = 12;
 
 void make_staging(Context &c)
 {
     HostStaging &h = c.staging;
     if (h.workers) return;
     const unsigned hw = std::thread::hardware_concurrency();
-    const int w = (int)std::max(1u, std::min(8u, hw / 2));
+    const int w = (int)std::max(1u, std::min(kStageWorkers, hw * 3 / 4));
     for (int i = 0; i < w; ++i) {
         cudaStream_t s;
         QB_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
@@ -252,7 +259,9 @@ void sync_check()
 {
     Context &c = ctx();
     QB_CUDA(cudaStreamSynchronize(c.stream));
-    if (!c.d_err) return;
+    // only kernels with bounded waits write the failure word
+    if (!c.d_err || !c.err_armed) return;
+    c.err_armed = false;
     int e = 0;
     QB_CUDA(cudaMemcpy(&e, c.d_err, sizeof(int), cudaMemcpyDeviceToHost));
     if (e) {

@@ -102,12 +102,13 @@ struct Context {
     std::string last_error;
 
     int *d_err = nullptr;            // kernel failure word (bounded waits)
+    mutable bool err_armed = false;  // a kernel that may set it was launched since it was read
     void *d_slots = nullptr;         // barrier slots of the resident solver loop
     HostStaging staging;             // made on the first large pageable upload
     Halo halo;                       // domain decomposition along t (halo.h)
     int global_dims[4] = {0, 0, 0, 0};  // the whole lattice (dims: this GPU's slab)
 
-    Launch launch() const { return Launch{stream, &g, d_err, halo.on ? &halo : nullptr}; }
+    Launch launch() const { return Launch{stream, &g, d_err, halo.on ? &halo : nullptr, &err_armed}; }
 };
 
 Context &ctx();

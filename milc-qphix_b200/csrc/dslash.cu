@@ -833,6 +833,7 @@ static void launch_variant(int variant, const DslashArgs<SV, SL> &a, const LinkS
     if (variant == 3) {
         if constexpr (std::is_same<SV, float>::value || std::is_same<SV, double>::value) {
             if (tile_ok<SV>(*L.g)) {
+                L.arm();
                 const TileShape ts = tile_shape<SV, SL, 0>(*L.g);
                 k_dslash_tile<SV, SL, 0><<<ts.grid, ts.block, ts.smem, L.stream>>>(
                     a, a.out, 0.0, const_cast<SolverState *>(st), nullptr, gate, 0, L.err, g_wait_limit);
@@ -844,6 +845,7 @@ static void launch_variant(int variant, const DslashArgs<SV, SL> &a, const LinkS
     if constexpr (!has_tma<SL>()) {
         if (variant == 2) variant = 1;
     } else if (variant == 2) {
+        L.arm();
         k_dslash_tma<SV, SL, 0><<<tma_grid<SV, SL, 0>(L.g->vh), TmaCfg<SL>::T, tma_smem_bytes<SL>(), L.stream>>>(
             a, static_cast<const char *>(ls.blk[cb]), a.out, 0.0, const_cast<SolverState *>(st), nullptr, gate, 0,
             L.err, g_wait_limit);
@@ -998,6 +1000,7 @@ static void launch_mdagm_variant(int variant, const DslashArgs<SV, SL> &a, const
     if (variant == 3) {
         if constexpr (std::is_same<SV, float>::value || std::is_same<SV, double>::value) {
             if (tile_ok<SV>(*L.g)) {
+                L.arm();
                 const TileShape ts = tile_shape<SV, SL, 1>(*L.g);
                 k_dslash_tile<SV, SL, 1><<<ts.grid, ts.block, ts.smem, L.stream>>>(a, pv, m4, st, partials, gate,
                                                                                    mode, L.err, g_wait_limit);
@@ -1009,6 +1012,7 @@ static void launch_mdagm_variant(int variant, const DslashArgs<SV, SL> &a, const
     if constexpr (!has_tma<SL>()) {
         if (variant == 2) variant = 1;
     } else if (variant == 2) {
+        L.arm();
         k_dslash_tma<SV, SL, 1><<<tma_grid<SV, SL, 1>(L.g->vh), TmaCfg<SL>::T, tma_smem_bytes<SL>(), L.stream>>>(
             a, static_cast<const char *>(ls.blk[cb]), pv, m4, st, partials, gate, mode, L.err, g_wait_limit);
         return;

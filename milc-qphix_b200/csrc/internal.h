@@ -176,6 +176,8 @@ struct Launch {
     const Geom *g;
     int *err;                     // device word set by a kernel whose bounded wait gave up
     const Halo *halo = nullptr;   // t faces through ghost buffers (domain decomposition)
+    bool *armed = nullptr;        // set by launches of kernels that may write err
+    void arm() const { if (armed) *armed = true; }
 };
 
 // out[cb] = D in[1-cb];  links = block of output parity cb

@@ -824,6 +824,7 @@ void launch_form(LoopArgs<SV, SL> &a, const Launch &L)
         ready = true;
     }
     check(cudaMemsetAsync(a.counter, 0, sizeof(unsigned), L.stream), "solver loop: memset");
+    L.arm();
     void *args[] = {&a};
     check(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(&k_solver_loop<SV, SL, MODE, MIR, PARTS>), dim3(nb),
                                       dim3(threads), args, smem, L.stream),

@@ -189,6 +189,7 @@ public:
             S.cond = handle_;
             S.iter_cap = S.iteration + (cap > 0 ? cap : 1);
             upload_state();
+            c.err_armed = true;  // (the graph may hold kernels with bounded waits)
             QB_CUDA(cudaGraphLaunch(exec_, c.stream));
             download_state();
             S.use_cond = 0;
