@@ -285,6 +285,7 @@ struct LoopRun {
     const LinkSet *links = nullptr;
     int parity = 0;
     VecBlock p, tmp, ttt, r, x;
+    VecBlock p2;            // scratch like p (small lattices; may be empty)
     double m4 = 0, delta2 = 0;
     SolverState *st = nullptr;
     void *slots = nullptr;  // solver_loop_slot_bytes() of device memory
@@ -294,6 +295,8 @@ struct LoopRun {
     MsHistEntry *hist_s = nullptr;
 };
 bool solver_loop_run(Prec pv, const LoopRun &q, const Launch &L);
+// whether solver_loop_run would use LoopRun::p2
+bool solver_loop_wants_p2(Prec pv, const Launch &L);
 size_t solver_loop_slot_bytes();
 // the loop would read mirrored links of this set as such (loop.cu has the rule)
 bool loop_wants_mirrored(const LinkSet &ls, int vh);

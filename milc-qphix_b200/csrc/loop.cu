@@ -34,14 +34,13 @@
 // and SM); smaller groups only spread lattices that would leave SMs idle.
 //
 // us per iteration of the kernels in the graph loop / here (one B200, m =
-// 0.02, reliable updates included): FP64 8^4 30.0 / 11.4, 12^3x24 39.0 /
-// 21.5, 16^3x32 69.4 / 59.8, 24^3x48 276 / 263; FP32 25.6 / 11.4, 29.9 /
-// 15.9, 45.5 / 31.1, 143.5 / 131.9; FP32 with 12-real Naik links 27.9 / 13.4,
-// 33.1 / 19.3, 47.3 / 36.0, 133.2 / 128.8; 16-bit links 27.6 / 13.2, 32.5 /
-// 18.8, 42.7 / 31.1, 104.6 / 102.4.  At 8^4 the four barriers are 7 us of
-// the iteration; at 24^3x48 the Dslash phases run at 5.6 TB/s of DRAM with
-// 45 % of the issue slots used, waiting for loads and at the groups'
-// barriers.
+// 0.02, reliable updates included): FP64 8^4 30.0 / 10.0, 12^3x24 39.0 /
+// 21.2, 16^3x32 69.4 / 59.4, 24^3x48 276 / 263; FP32 25.6 / 9.5, 29.9 /
+// 15.2, 45.5 / 31.2, 143.5 / 130.0; FP32 with 12-real Naik links 27.9 / 11.9,
+// 33.1 / 18.7, 47.3 / 34.9, 133.2 / 127.4; 16-bit links 27.6 / 12.0, 32.5 /
+// 18.4, 42.7 / 30.5, 104.6 / 99.8.  At 8^4 the barriers are half of the
+// iteration; at 24^3x48 the Dslash phases run at 5.6 TB/s of DRAM with 45 %
+// of the issue slots used, waiting for loads and at the groups' barriers.
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -86,6 +85,7 @@ struct LoopArgs {
     LinkView<SL> links[2];  // by output parity
     int parity;             // parity of p, ttt, r, x
     VecView<SV> p, tmp, ttt, r;
+    VecView<SV> p2;         // second buffer of the direction (k_small_loop)
     void *x;                // CG: the solution (FP32 under 16-bit vectors)
     double m4, delta2;
     SolverState *st;
@@ -208,6 +208,25 @@ __device__ __forceinline__ void ld_vec(const VecView<__half> &f, int j, float v[
     VecView<__half>::unpack(f.p[j], v);
 }
 
+// The Dslash input r + b p of a direction that is not stored yet (`first`: p
+// itself)
+template <typename SV>
+struct SumIn {
+    VecView<SV> p, r;
+    SV b;
+    bool first;
+    __device__ __forceinline__ SV at(SV pv, SV rv) const { return first ? pv : fma_(b, pv, rv); }
+};
+template <typename SV>
+__device__ __forceinline__ void ld_vec(const SumIn<SV> &f, int j, SV v[6])
+{
+    SV q[6];
+    ld_vec(f.p, j, v);
+    ld_vec(f.r, j, q);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) v[k] = f.at(v[k], q[k]);
+}
+
 // What a thread of part (direction d, hop 1 + 2h) keeps for all its sites
 struct PartGeom {
     int n, str;  // extent and stride of d
@@ -233,9 +252,9 @@ __device__ __forceinline__ void part_neighbors(const PartGeom &q, const SiteCoor
 // of site j.  lk: the links of the output parity, lo: of the other.  Mirrored: the
 // backward link is read as the forward link of its own site b (lo), where
 // the caller's backward links are exactly those (LinkSet::mirrored).
-template <bool MIR>
+template <bool MIR, typename In>
 __device__ __forceinline__ void part_dslash(const LinkView<double> &lk, const LinkView<double> &lo,
-                                            const VecView<double> &in, int d, int h, int j, int f, int b,
+                                            const In &in, int d, int h, int j, int f, int b,
                                             double acc[6])
 {
     double vf[6], vb[6], u[18], w[18];
@@ -257,8 +276,8 @@ __device__ __forceinline__ void part_dslash(const LinkView<double> &lk, const Li
     mv_adj_sub_fma(acc, w, vb);
 }
 
-template <bool MIR, typename SV, typename SL>
-__device__ __forceinline__ void part_dslash(const LinkView<SL> &lk, const LinkView<SL> &lo, const VecView<SV> &in,
+template <bool MIR, typename In, typename SL>
+__device__ __forceinline__ void part_dslash(const LinkView<SL> &lk, const LinkView<SL> &lo, const In &in,
                                             int d, int h, int j, int f, int b, float acc[6])
 {
     float vf[6], vb[6], u[36];
@@ -392,13 +411,14 @@ __device__ __forceinline__ GroupPlace group_place(const LoopArgs<SV, SL> &a)
     return p;
 }
 
-// One tile: out = D in (+ m4 p, with the products p.out added to dot) at the
-// group's sites j0 .. j0 + sg - 1 of parity cb.  `buf`: 6 reals per thread of
+// One tile: out = D in (+ m4 p, with the products p.out added to dot; `own`
+// gives component c of p at site j) at the group's sites j0 .. j0 + sg - 1 of
+// parity cb.  `buf`: 6 reals per thread of
 // the group; the caller alternates two of them, so a thread that reaches the
 // next tile's barrier has read the buffer of the tile before.
-template <int PARTS, bool MDAGM, bool MIR, typename SV, typename SL, typename A>
+template <int PARTS, bool MDAGM, bool MIR, typename SV, typename SL, typename In, typename A, typename Own>
 __device__ __forceinline__ void tile_dslash(const LoopArgs<SV, SL> &a, const GroupPlace &p, int j0, int cb,
-                                            const VecView<SV> &in, const VecView<SV> &out, A *buf, double &dot)
+                                            const In &in, const VecView<SV> &out, A *buf, double &dot, Own own)
 {
     const int j = j0 + p.i, vh = a.g.vh, sg = a.sg, part = p.part;
     SiteCoords s;
@@ -431,7 +451,7 @@ __device__ __forceinline__ void tile_dslash(const LoopArgs<SV, SL> &a, const Gro
     }
     cx_t<A> pv;
     if constexpr (MDAGM && !std::is_same<SV, __half>::value)
-        if (part < 3) pv = a.p.p[part * vh + j];
+        if (part < 3) pv = own(part, j);
 #pragma unroll
     for (int k = 0; k < 6; ++k) buf[(part * 6 + k) * sg + p.i] = acc[k];
     group_sync(1 + p.grp, p.gthreads);
@@ -474,15 +494,16 @@ __device__ __forceinline__ void tile_dslash(const LoopArgs<SV, SL> &a, const Gro
 }
 
 // out = D in (+ m4 p) over the lattice, the groups striding over the tiles
-template <int PARTS, bool MDAGM, bool MIR, typename SV, typename SL, typename A>
-__device__ __forceinline__ void phase_dslash(const LoopArgs<SV, SL> &a, const GroupPlace &p, int cb,
-                                             const VecView<SV> &in, const VecView<SV> &out, A *comb, double &dot)
+template <int PARTS, bool MDAGM, bool MIR, typename SV, typename SL, typename In, typename A, typename Own>
+__device__ __forceinline__ void phase_dslash(const LoopArgs<SV, SL> &a, const GroupPlace &p, int cb, const In &in,
+                                             const VecView<SV> &out, A *comb, double &dot, Own own)
 {
     if (p.grp >= a.groups) return;
     const int per = a.groups * a.sg;
     unsigned k = 0;
     for (int j0 = blockIdx.x * per + p.grp * a.sg; j0 < a.g.vh; j0 += gridDim.x * per, ++k)
-        tile_dslash<PARTS, MDAGM, MIR>(a, p, j0, cb, in, out, comb + ((size_t)p.grp * 2 + (k & 1)) * 6 * p.gthreads, dot);
+        tile_dslash<PARTS, MDAGM, MIR>(a, p, j0, cb, in, out, comb + ((size_t)p.grp * 2 + (k & 1)) * 6 * p.gthreads, dot,
+                                       own);
 }
 
 // 16-byte words of the flat element-wise phases
@@ -608,24 +629,29 @@ __device__ __forceinline__ void phase_shifts(int vh, const SolverState &S, VecBl
     }
 }
 
-// the deferred form (k_ms_defer's arithmetic): r and the shifts' scalars into
-// the iteration's slot, p_low = z r + a p_low
+// the deferred form (k_ms_defer's arithmetic): r (phase_defer) and the shifts'
+// scalars (defer_scalars) into the iteration's slot, p_low = z r + a p_low
+__device__ __forceinline__ void defer_scalars(const SolverState &S, int slot, MsHistEntry *hs, int n)
+{
+    const int it = S.iteration, nn = S.num_now;
+    const bool conv = S.converged != 0;
+    for (int k = threadIdx.x; k < n; k += blockDim.x) {
+        MsHistEntry e;
+        e.b = S.beta_i[k];
+        e.a = S.alpha[k];
+        e.z = S.zeta_ip1[k];
+        const int sd = S.shift_done_at[k];
+        e.upd = k >= nn || sd < it ? 0 : (1 | (!conv && sd != it ? 2 : 0));
+        hs[(size_t)slot * n + k] = e;
+    }
+}
+
 __device__ __forceinline__ void phase_defer(int vh, SolverState &S, const VecView<float> &p, const VecView<float> &r,
                                             float2 *hist, MsHistEntry *hs, int n)
 {
-    const int it = S.iteration, slot = it - S.ms_seg_start - 1, jl = S.j_low, nn = S.num_now;
+    const int slot = S.iteration - S.ms_seg_start - 1, jl = S.j_low;
     const bool conv = S.converged != 0;
-    if (blockIdx.x == 0) {
-        for (int k = threadIdx.x; k < n; k += blockDim.x) {
-            MsHistEntry e;
-            e.b = S.beta_i[k];
-            e.a = S.alpha[k];
-            e.z = S.zeta_ip1[k];
-            const int sd = S.shift_done_at[k];
-            e.upd = k >= nn || sd < it ? 0 : (1 | (!conv && sd != it ? 2 : 0));
-            hs[(size_t)slot * n + k] = e;
-        }
-    }
+    if (blockIdx.x == 0) defer_scalars(S, slot, hs, n);
     const int n4 = 6 * vh / 4, step = gridDim.x * blockDim.x;
     float4 *h = reinterpret_cast<float4 *>(hist + (size_t)slot * 3 * vh);
     const float ak = (float)S.alpha[jl];
@@ -647,6 +673,14 @@ __device__ __forceinline__ void phase_defer(int vh, SolverState &S, const VecVie
     }
 }
 
+__device__ __forceinline__ void load_state(SolverState &to, const SolverState *from)
+{
+    const int nw = sizeof(SolverState) / sizeof(int);
+    const int *src = reinterpret_cast<const int *>(from);
+    int *dst = reinterpret_cast<int *>(&to);
+    for (int i = threadIdx.x; i < nw; i += blockDim.x) dst[i] = src[i];
+}
+
 template <typename SV, typename SL, int MODE, bool MIR, int PARTS>
 __global__ void __launch_bounds__(LoopThreads<SV>::value, 1) k_solver_loop(const LoopArgs<SV, SL> a)
 {
@@ -656,10 +690,7 @@ __global__ void __launch_bounds__(LoopThreads<SV>::value, 1) k_solver_loop(const
     A *comb = reinterpret_cast<A *>(dyn);
     SolverState &S = sh.st;
     {
-        const int nw = sizeof(SolverState) / sizeof(int);
-        const int *src = reinterpret_cast<const int *>(a.st);
-        int *dst = reinterpret_cast<int *>(&sh.st);
-        for (int i = threadIdx.x; i < nw; i += blockDim.x) dst[i] = src[i];
+        load_state(sh.st, a.st);
         if (threadIdx.x == 0) sh.fail = 0;
     }
     __syncthreads();
@@ -671,9 +702,13 @@ __global__ void __launch_bounds__(LoopThreads<SV>::value, 1) k_solver_loop(const
     bool ok = true;
     for (;;) {
         double v = 0.0, tot;
-        phase_dslash<PARTS, false, MIR>(a, place, 1 - par, a.p, a.tmp, comb, v);
+        const auto own = [&](int c, int j) {
+            if constexpr (std::is_same<SV, __half>::value) return cx_t<A>();
+            else return a.p.p[c * vh + j];
+        };
+        phase_dslash<PARTS, false, MIR>(a, place, 1 - par, a.p, a.tmp, comb, v, [] (int, int) { return cx_t<A>(); });
         if (!(ok = grid_wait(sh, bar))) break;
-        phase_dslash<PARTS, true, MIR>(a, place, par, a.tmp, a.ttt, comb, v);
+        phase_dslash<PARTS, true, MIR>(a, place, par, a.tmp, a.ttt, comb, v, own);
         if (!(ok = grid_sum(v, tot, sh, bar))) break;
         if (warp0) FinMdagm{&S, kMs ? 1 : 0}(&tot, (int)threadIdx.x);
         __syncthreads();
@@ -748,11 +783,131 @@ __global__ void __launch_bounds__(LoopThreads<SV>::value, 1) k_solver_loop(const
     }
     if (blockIdx.x == 0) {
         __syncthreads();
-        const int nw = sizeof(SolverState) / sizeof(int);
-        const int *src = reinterpret_cast<const int *>(&sh.st);
-        int *dst = reinterpret_cast<int *>(a.st);
-        for (int i = threadIdx.x; i < nw; i += blockDim.x) dst[i] = src[i];
+        load_state(*a.st, &sh.st);
     }
+}
+
+// The loop of a lattice whose sites all fit the grid at once, bound by its
+// barriers: three per iteration instead of four.  The direction p = r + b p is
+// not stored by a phase of its own; the first half of M^dag M forms it at the
+// neighbours it gathers, the second half at its own sites, storing it in the
+// other of two buffers (every use has the same operands, hence the same
+// bits):
+//   1  tmp = D (r + b p)                          | barrier
+//   2  p' = r + b p, ttt = D tmp + m4 p', p'.ttt  | barrier with sum
+//   3  r += a ttt, x += a p', |r|^2 (multi-shift: r into its slot) | barrier with sum
+// Twice the gathered bytes in phase 1, but no barrier and no pass for the
+// direction.  us per iteration with four phases / three: 8^4 FP64 11.4 / 10.0,
+// FP32 11.4 / 9.5, 12-real 13.4 / 11.9.
+template <typename SV> struct SmallThreads { static constexpr int value = 512; };
+template <> struct SmallThreads<double> { static constexpr int value = 256; };
+
+template <typename SV, typename SL, int MODE>
+__global__ void __launch_bounds__(SmallThreads<SV>::value, 1) k_small_loop(const LoopArgs<SV, SL> a)
+{
+    using F = FlatWord<SV>;
+    using W = typename F::type;
+    __shared__ LoopShared sh;
+    extern __shared__ __align__(16) unsigned char dyn[];
+    SV *comb = reinterpret_cast<SV *>(dyn);
+    SolverState &S = sh.st;
+    load_state(sh.st, a.st);
+    if (threadIdx.x == 0) sh.fail = 0;
+    __syncthreads();
+    const int vh = a.g.vh, par = a.parity;
+    const bool warp0 = threadIdx.x < 32;
+    constexpr bool kMs = MODE == kLoopMsDefer;
+    LoopBarrier bar{a.counter, a.partials, 0};
+    const GroupPlace place = group_place<8>(a);
+    const int n = 6 * vh / F::n, flat0 = blockIdx.x * blockDim.x + threadIdx.x, flat_step = gridDim.x * blockDim.x;
+    VecView<SV> cur = a.p, other = a.p2;
+    bool ok = true, first = true;
+    SV b = SV(0);
+    for (;;) {
+        double v = 0.0, tot;
+        const SumIn<SV> in{cur, a.r, b, first};
+        phase_dslash<8, false, false>(a, place, 1 - par, in, a.tmp, comb, v, [](int, int) { return cx_t<SV>(); });
+        if (!(ok = grid_wait(sh, bar))) break;
+        phase_dslash<8, true, false>(a, place, par, a.tmp, a.ttt, comb, v, [&](int c, int j) {
+            cx_t<SV> z = in.p.p[c * vh + j];
+            const cx_t<SV> q = in.r.p[c * vh + j];
+            z.x = in.at(z.x, q.x);
+            z.y = in.at(z.y, q.y);
+            other.p[c * vh + j] = z;
+            return z;
+        });
+        if (!(ok = grid_sum(v, tot, sh, bar))) break;
+        const VecView<SV> keep = cur;
+        cur = other;
+        other = keep;
+        first = false;
+        if (warp0) FinMdagm{&S, kMs ? 1 : 0}(&tot, (int)threadIdx.x);
+        __syncthreads();
+        const SV s = (SV)(kMs ? S.beta_i[S.j_low] : S.a);
+        const int slot = kMs ? S.iteration - S.ms_seg_start - 1 : 0;
+        const bool slot_ok = !kMs || (slot >= 0 && slot < S.ms_seg_cap);
+        W *h = kMs && slot_ok ? reinterpret_cast<W *>(a.hist + (size_t)slot * 3 * vh) : nullptr;
+        v = 0.0;
+        for (int i = flat0; i < n; i += flat_step) {
+            SV rv[F::n], tv[F::n];
+            F::get(reinterpret_cast<const W *>(a.r.p)[i], rv);
+            F::get(reinterpret_cast<const W *>(a.ttt.p)[i], tv);
+            if constexpr (!kMs) {
+                SV xv[F::n], pv[F::n];
+                F::get(static_cast<const W *>(a.x)[i], xv);
+                F::get(reinterpret_cast<const W *>(cur.p)[i], pv);
+#pragma unroll
+                for (int e = 0; e < F::n; ++e) xv[e] = xv[e] + s * pv[e];
+                static_cast<W *>(a.x)[i] = F::make(xv);
+            }
+#pragma unroll
+            for (int e = 0; e < F::n; ++e) {
+                rv[e] = rv[e] + s * tv[e];
+                v += (double)(rv[e] * rv[e]);
+            }
+            const W w = F::make(rv);
+            reinterpret_cast<W *>(a.r.p)[i] = w;
+            if (h) h[i] = w;
+        }
+        if (!(ok = grid_sum(v, tot, sh, bar))) break;
+        if constexpr (MODE == kLoopCg) {
+            if (threadIdx.x == 0) FinCgUpdate{&S, 0, false, 1.0}(&tot);
+        } else if constexpr (MODE == kLoopMx) {
+            if (threadIdx.x == 0) FinMx{&S, 0, a.delta2}(&tot);
+        } else {
+            if (warp0) FinMsResidual{&S, 0}(&tot, (int)threadIdx.x);
+        }
+        __syncthreads();
+        if constexpr (kMs) {
+            if (!slot_ok) {  // uniform over the grid
+                if (threadIdx.x == 0) {
+                    S.error = 3;
+                    S.stop_at = 0;
+                }
+                __syncthreads();
+            } else if (blockIdx.x == 0) {
+                defer_scalars(S, slot, a.hist_s, a.n);
+            }
+        }
+        b = (SV)(kMs ? S.alpha[S.j_low] : S.b);
+        if (S.stop_at != INT_MAX) break;
+    }
+    if (!ok) {
+        if (threadIdx.x == 0) atomicExch(a.err, 1);
+        return;
+    }
+    // the direction as the four-phase loop leaves it, in the caller's buffer
+    // (all reads of the last phases are behind the last barrier)
+    const bool dir = kMs ? S.converged == 0 : S.skip_axpy == 0;
+    for (int i = flat0; i < n; i += flat_step) {
+        SV pv[F::n], rv[F::n];
+        F::get(reinterpret_cast<const W *>(cur.p)[i], pv);
+        F::get(reinterpret_cast<const W *>(a.r.p)[i], rv);
+#pragma unroll
+        for (int e = 0; e < F::n; ++e) pv[e] = dir ? fma_(b, pv[e], rv[e]) : pv[e];
+        reinterpret_cast<W *>(a.p.p)[i] = F::make(pv);
+    }
+    if (blockIdx.x == 0) load_state(*a.st, &sh.st);
 }
 
 void check(cudaError_t e, const char *what)
@@ -792,22 +947,21 @@ FastDiv fast_div(int n)
     return d;
 }
 
-template <typename SV, typename SL, int MODE, bool MIR, int PARTS>
-void launch_form(LoopArgs<SV, SL> &a, const Launch &L)
+// one block per SM, groups of 32 sites; a lattice with fewer groups than SMs
+// takes smaller ones (vh is a multiple of 128)
+template <typename SV, typename SL, typename K>
+void launch_kernel(LoopArgs<SV, SL> &a, K kernel, int parts, int max_threads, const Launch &L)
 {
     using A = typename Acc<SV>::type;
-    const int vh = L.g->vh;
-    // one block per SM, groups of 32 sites; a lattice with fewer groups than
-    // SMs takes smaller ones (vh is a multiple of 128)
-    const int sms = sm_count();
+    const int vh = L.g->vh, sms = sm_count();
     a.sg = 32;
     a.lg_sg = 5;
     while (a.sg > 4 && vh / a.sg < sms) {
         a.sg >>= 1;
         --a.lg_sg;
     }
-    const int ngroups = vh / a.sg, gthreads = PARTS * a.sg;
-    a.groups = std::min(LoopThreads<SV>::value / gthreads, (ngroups + sms - 1) / sms);
+    const int ngroups = vh / a.sg, gthreads = parts * a.sg;
+    a.groups = std::min(max_threads / gthreads, (ngroups + sms - 1) / sms);
     a.groups = std::min(a.groups, 8);  // one hardware barrier each
     const int nb = std::min(sms, (ngroups + a.groups - 1) / a.groups);
     // every block has a thread per partial sum
@@ -816,19 +970,21 @@ void launch_form(LoopArgs<SV, SL> &a, const Launch &L)
     a.dx = fast_div(L.g->nxh);
     a.dy = fast_div(L.g->ny);
     a.dz = fast_div(L.g->nz);
-    static bool ready = false;
-    if (!ready) {
-        check(cudaFuncSetAttribute(k_solver_loop<SV, SL, MODE, MIR, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)(LoopThreads<SV>::value * 12 * sizeof(A))),
-              "solver loop: shared memory");
-        ready = true;
-    }
+    check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)(max_threads * 12 * sizeof(A))),
+          "solver loop: shared memory");
     check(cudaMemsetAsync(a.counter, 0, sizeof(unsigned), L.stream), "solver loop: memset");
     L.arm();
     void *args[] = {&a};
-    check(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(&k_solver_loop<SV, SL, MODE, MIR, PARTS>), dim3(nb),
-                                      dim3(threads), args, smem, L.stream),
+    check(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kernel), dim3(nb), dim3(threads), args, smem,
+                                      L.stream),
           "solver loop: launch");
+}
+
+template <typename SV, typename SL, int MODE, bool MIR, int PARTS>
+void launch_form(LoopArgs<SV, SL> &a, const Launch &L)
+{
+    launch_kernel<SV, SL>(a, k_solver_loop<SV, SL, MODE, MIR, PARTS>, PARTS, LoopThreads<SV>::value, L);
 }
 
 template <typename SV, typename SL, int MODE>
@@ -855,6 +1011,13 @@ bool launch(const LoopRun &q, const Launch &L)
     a.ps = q.ps;
     a.hist = static_cast<float2 *>(q.hist.data);
     a.hist_s = q.hist_s;
+    if constexpr (MODE != kLoopMs && !std::is_same<SV, __half>::value) {
+        if (q.p2.data && vh <= sm_count() * (SmallThreads<SV>::value / 8)) {
+            a.p2 = view<SV>(q.p2, vh);
+            launch_kernel<SV, SL>(a, k_small_loop<SV, SL, MODE>, 8, SmallThreads<SV>::value, L);
+            return true;
+        }
+    }
     const bool eight = vh <= LoopThreads<SV>::eight_parts;
     const bool mir = q.links->mirrored == 1 && loop_wants_mirrored(*q.links, vh);
     if (mir) {
@@ -882,6 +1045,13 @@ bool loop_wants_mirrored(const LinkSet &ls, int vh)
 {
     const size_t bytes = loop_link_bytes(ls, vh);
     return bytes >= ((size_t)64 << 20) && bytes <= ((size_t)152 << 20);
+}
+
+bool solver_loop_wants_p2(Prec pv, const Launch &L)
+{
+    return pv == Prec::Double   ? L.g->vh <= sm_count() * (SmallThreads<double>::value / 8)
+           : pv == Prec::Single ? L.g->vh <= sm_count() * (SmallThreads<float>::value / 8)
+                                : false;
 }
 
 bool solver_loop_run(Prec pv, const LoopRun &q, const Launch &L)

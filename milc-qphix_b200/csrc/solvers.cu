@@ -302,6 +302,7 @@ int cg_reference(Prec P, const LinkSet &ls, SolveArgs &A)
 
     Ws ws;
     VecBlock ttt = ws.get(P), tmp = ws.get(P), cg_p = ws.get(P), resid = ws.get(P);
+    VecBlock cg_p2 = solver_loop_wants_p2(P, L) ? ws.get(P) : VecBlock{};
     info->final_sec = wall_seconds();
     info->final_flop = 0.;
     TimedLaunches tl(c.kernel_timing);
@@ -386,7 +387,7 @@ int cg_reference(Prec P, const LinkSet &ls, SolveArgs &A)
             lr.mode = kLoopCg;
             lr.links = &ls;
             lr.parity = parity;
-            lr.p = cg_p; lr.tmp = tmp; lr.ttt = ttt; lr.r = resid; lr.x = t_dest;
+            lr.p = cg_p; lr.p2 = cg_p2; lr.tmp = tmp; lr.ttt = ttt; lr.r = resid; lr.x = t_dest;
             lr.m4 = -msq_x4;
             loop.run(
                 [&](int k) {
@@ -516,6 +517,7 @@ MixedResult mixed_pass(Prec ps, const LinkSet &ls64, const LinkSet &lss, const L
     VecBlock tmp64 = ws.get(Prec::Double), ttt64 = ws.get(Prec::Double), r64 = ws.get(Prec::Double);
     // the partial solution x_s is FP32 under a 16-bit inner solve
     VecBlock xs = ws.get(inner_x_prec(ps)), rs = ws.get(ps), pv = ws.get(ps), tmps = ws.get(ps), ttts = ws.get(ps);
+    VecBlock pv2 = solver_loop_wants_p2(ps, L) ? ws.get(ps) : VecBlock{};
 
     auto true_residual = [&]() {
         S.msq_x4 = m4;
@@ -558,7 +560,7 @@ MixedResult mixed_pass(Prec ps, const LinkSet &ls64, const LinkSet &lss, const L
         lr.mode = kLoopMx;
         lr.links = ls_cur;
         lr.parity = parity;
-        lr.p = pv; lr.tmp = tmps; lr.ttt = ttts; lr.r = rs; lr.x = xs;
+        lr.p = pv; lr.p2 = pv2; lr.tmp = tmps; lr.ttt = ttts; lr.r = rs; lr.x = xs;
         lr.m4 = -m4;
         lr.delta2 = delta2;
         loop.run(
@@ -613,6 +615,7 @@ MixedResult mixed_pass(Prec ps, const LinkSet &ls64, const LinkSet &lss, const L
             tmps = ws.get(Prec::Single);
             ttts = ws.get(Prec::Single);
             ps = Prec::Single;
+            if (!pv2.data && solver_loop_wants_p2(ps, L)) pv2 = ws.get(ps);
             ls_cur = ls_up;
             stalled = 0;
             out.escalated = 1;
@@ -861,6 +864,8 @@ MsPass ms_pass(Prec p, Prec xp, const LinkSet &ls, VecBlock src, std::vector<Vec
     const double m4 = round_prec(-1.0 * offset_low, single);
     double size_prev = out.rsq;
     dslash_prepare(p, ls, L);
+    Ws ws2;
+    VecBlock p2 = df && solver_loop_wants_p2(p, L) ? ws2.get(p) : VecBlock{};
     IterLoop loop;
     int ru_stalls = 0;
     double t_run = 0, t_flush = 0, t_ru = 0;  // verbose: host-side phase times
@@ -871,7 +876,7 @@ MsPass ms_pass(Prec p, Prec xp, const LinkSet &ls, VecBlock src, std::vector<Vec
         lr.mode = df ? kLoopMsDefer : kLoopMs;
         lr.links = &ls;
         lr.parity = parity;
-        lr.p = pm[j_low]; lr.tmp = tmp; lr.ttt = ttt; lr.r = resid;
+        lr.p = pm[j_low]; lr.p2 = p2; lr.tmp = tmp; lr.ttt = ttt; lr.r = resid;
         lr.m4 = m4;
         lr.n = n;
         lr.xs = d_x; lr.ps = d_p;
