@@ -192,14 +192,20 @@ struct GaugeView {
 //  * the block indices of the wrapped coordinates x - 2 .. x + 2 along each
 //    axis are computed once into shared memory;
 //  * adjoints are taken in the product, by a branch the whole warp takes;
-//  * the staple sum S, used seven times per link, is in shared memory.
+//  * the staple sum S, used seven times per link, is in shared memory, and in
+//    FP64 so is X, used 37 times (24^3x48, one checkerboard: 3.48 ms against
+//    3.76 ms with X in registers at three blocks per SM both, 4.80 ms at four
+//    blocks with spills; FP32 2.17 ms with X in registers at five blocks,
+//    2.25 ms with X in shared memory at six).
 constexpr int kGfThreads = 128;
+template <typename R> constexpr bool kGfSharedX = std::is_same<R, double>::value;
 template <typename R> struct GfMinBlocks { static constexpr int value = 5; };
 template <> struct GfMinBlocks<double> { static constexpr int value = 3; };
 
 template <typename R>
 struct GfShared {
-    R acc[18][kGfThreads];
+    R acc[18][kGfThreads];  // S
+    R x[kGfSharedX<R> ? 18 : 1][kGfThreads];  // X
     int idx[4][5][kGfThreads];  // by axis and displacement + 2
 };
 
@@ -226,13 +232,20 @@ __device__ __forceinline__ void gf_apply(GfShared<R> &sh, unsigned op, const R u
     } else if (op == kFold) {
 #pragma unroll
         for (int r = 0; r < 3; ++r) {
-            R t[6];
-            mm_row<ADJ>(X + 6 * r, u, t);
+            R a[6], t[6];
 #pragma unroll
             for (int k = 0; k < 6; ++k) {
-                sh.acc[6 * r + k][threadIdx.x] += t[k];
-                X[6 * r + k] = R(0);
+                if constexpr (kGfSharedX<R>) {
+                    a[k] = sh.x[6 * r + k][threadIdx.x];
+                    sh.x[6 * r + k][threadIdx.x] = R(0);
+                } else {
+                    a[k] = X[6 * r + k];
+                    X[6 * r + k] = R(0);
+                }
             }
+            mm_row<ADJ>(a, u, t);
+#pragma unroll
+            for (int k = 0; k < 6; ++k) sh.acc[6 * r + k][threadIdx.x] += t[k];
         }
     } else {
         const bool mix = op == kMix;
@@ -252,6 +265,7 @@ template <typename R>
 __global__ void __launch_bounds__(kGfThreads, GfMinBlocks<R>::value)
 k_gauge_force(GaugeView<R> U, cx_t<R> *mom, int cb, R eps, R c0, R c1, R c2, int mask)
 {
+    static_assert(sizeof(GfShared<R>) <= 48 * 1024, "static shared memory");
     __shared__ GfShared<R> sh;
     const Geom &g = U.g;
     const int idx = blockIdx.x * blockDim.x + threadIdx.x, tid = threadIdx.x;
@@ -271,8 +285,10 @@ k_gauge_force(GaugeView<R> U, cx_t<R> *mom, int cb, R eps, R c0, R c1, R c2, int
     R M[18], X[18], ua[18], ub[18];
 #pragma unroll
     for (int i = 0; i < 18; ++i) {
-        X[i] = M[i] = R(0);
+        M[i] = R(0);
         sh.acc[i][tid] = R(0);
+        if constexpr (kGfSharedX<R>) sh.x[i][tid] = R(0);
+        else X[i] = R(0);
     }
     const unsigned *prog = c_gf_program[mask][mu];
     const int n = c_gf_length[mask][mu];
@@ -283,7 +299,10 @@ k_gauge_force(GaugeView<R> U, cx_t<R> *mom, int cb, R eps, R c0, R c1, R c2, int
         if (add) {
             const R c = add == 1 ? c0 : add == 2 ? c1 : add == 3 ? c2 : R(1);
 #pragma unroll
-            for (int k = 0; k < 18; ++k) X[k] = fma_(c, M[k], X[k]);
+            for (int k = 0; k < 18; ++k) {
+                if constexpr (kGfSharedX<R>) sh.x[k][tid] = fma_(c, M[k], sh.x[k][tid]);
+                else X[k] = fma_(c, M[k], X[k]);
+            }
         }
     };
     if (n) gf_load(U, sh, cb, prog[0], ua);
@@ -297,7 +316,7 @@ k_gauge_force(GaugeView<R> U, cx_t<R> *mom, int cb, R eps, R c0, R c1, R c2, int
         }
     }
 #pragma unroll
-    for (int i = 0; i < 18; ++i) X[i] = sh.acc[i][tid];
+    for (int i = 0; i < 18; ++i) ua[i] = sh.acc[i][tid];
     {
         const cx_t<R> *p = U.b[cb] + (size_t)mu * 9 * g.vh + j;
 #pragma unroll
@@ -307,7 +326,7 @@ k_gauge_force(GaugeView<R> U, cx_t<R> *mom, int cb, R eps, R c0, R c1, R c2, int
             M[2 * k + 1] = z.y;
         }
     }
-    mm_inplace<false>(M, X);  // W = U S
+    mm_inplace<false>(M, ua);  // W = U S
     // TA(W) = (W - W^dag)/2 - tr(W - W^dag)/6
     const R tr = (M[1] + M[9] + M[17]) * (R(1) / R(3));  // imaginary part of tr(W - W^dag)/2 / 3
     cx_t<R> *m = mom + (size_t)mu * 9 * g.vh + j;
