@@ -948,9 +948,10 @@ FastDiv fast_div(int n)
 }
 
 // one block per SM, groups of 32 sites; a lattice with fewer groups than SMs
-// takes smaller ones (vh is a multiple of 128)
+// takes smaller ones (vh is a multiple of 128).  False when the blocks cannot
+// all be resident (a process with a share of the SMs).
 template <typename SV, typename SL, typename K>
-void launch_kernel(LoopArgs<SV, SL> &a, K kernel, int parts, int max_threads, const Launch &L)
+bool launch_kernel(LoopArgs<SV, SL> &a, K kernel, int parts, int max_threads, const Launch &L)
 {
     using A = typename Acc<SV>::type;
     const int vh = L.g->vh, sms = sm_count();
@@ -976,15 +977,20 @@ void launch_kernel(LoopArgs<SV, SL> &a, K kernel, int parts, int max_threads, co
     check(cudaMemsetAsync(a.counter, 0, sizeof(unsigned), L.stream), "solver loop: memset");
     L.arm();
     void *args[] = {&a};
-    check(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kernel), dim3(nb), dim3(threads), args, smem,
-                                      L.stream),
-          "solver loop: launch");
+    const cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kernel), dim3(nb), dim3(threads),
+                                                      args, smem, L.stream);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {
+        (void)cudaGetLastError();  // not sticky
+        return false;
+    }
+    check(e, "solver loop: launch");
+    return true;
 }
 
 template <typename SV, typename SL, int MODE, bool MIR, int PARTS>
-void launch_form(LoopArgs<SV, SL> &a, const Launch &L)
+bool launch_form(LoopArgs<SV, SL> &a, const Launch &L)
 {
-    launch_kernel<SV, SL>(a, k_solver_loop<SV, SL, MODE, MIR, PARTS>, PARTS, LoopThreads<SV>::value, L);
+    return launch_kernel<SV, SL>(a, k_solver_loop<SV, SL, MODE, MIR, PARTS>, PARTS, LoopThreads<SV>::value, L);
 }
 
 template <typename SV, typename SL, int MODE>
@@ -1014,20 +1020,13 @@ bool launch(const LoopRun &q, const Launch &L)
     if constexpr (MODE != kLoopMs && !std::is_same<SV, __half>::value) {
         if (q.p2.data && vh <= sm_count() * (SmallThreads<SV>::value / 8)) {
             a.p2 = view<SV>(q.p2, vh);
-            launch_kernel<SV, SL>(a, k_small_loop<SV, SL, MODE>, 8, SmallThreads<SV>::value, L);
-            return true;
+            return launch_kernel<SV, SL>(a, k_small_loop<SV, SL, MODE>, 8, SmallThreads<SV>::value, L);
         }
     }
     const bool eight = vh <= LoopThreads<SV>::eight_parts;
-    const bool mir = q.links->mirrored == 1 && loop_wants_mirrored(*q.links, vh);
-    if (mir) {
-        if (eight) launch_form<SV, SL, MODE, true, 8>(a, L);
-        else launch_form<SV, SL, MODE, true, 4>(a, L);
-    } else {
-        if (eight) launch_form<SV, SL, MODE, false, 8>(a, L);
-        else launch_form<SV, SL, MODE, false, 4>(a, L);
-    }
-    return true;
+    if (q.links->mirrored == 1 && loop_wants_mirrored(*q.links, vh))
+        return eight ? launch_form<SV, SL, MODE, true, 8>(a, L) : launch_form<SV, SL, MODE, true, 4>(a, L);
+    return eight ? launch_form<SV, SL, MODE, false, 8>(a, L) : launch_form<SV, SL, MODE, false, 4>(a, L);
 }
 
 }  // namespace

@@ -1,7 +1,8 @@
 // Solver drivers: CG and multi-shift CG with the reference's control flow,
 // and their mixed-precision counterparts.
 //
-// The iteration bodies run as device kernels with every scalar (rsq, pkp,
+// The iterations of a solver phase run in one resident kernel (loop.cu) or,
+// where the phase has no such form, as device kernels, with every scalar (rsq, pkp,
 // a, b, the shift recurrences) kept in a device-resident SolverState; the
 // host enqueues chunks of iterations and reads the state once per chunk.
 // Each kernel of iteration k of a chunk returns immediately when an earlier
@@ -136,6 +137,8 @@ int next_chunk(int current, double size_prev, double size_now, int done, double 
 // Runs the device iterations of one solver phase until the device stops.
 // `enqueue(gate)` enqueues one iteration; `next(chunk, it0)` sizes the next
 // chunk from the host mirror S.
+//  * Resident mode (loop.cu): the phase is one cooperative launch.  On one
+//    GPU, for the phases that have this form.
 //  * Graph mode: the iteration is captured once (per phase configuration)
 //    into the body of a CUDA-graph while loop; the update kernel's last
 //    block clears the loop condition when the stop test fires, so a whole
