@@ -168,3 +168,27 @@ def test_force_autograd_matches_finite_differences(gpu):
         an = float(fat.grad.numpy() @ df + lng.grad.numpy() @ dl)
         worst = max(worst, abs(fd - an) / abs(an))
     assert worst < 1e-6, worst
+
+
+@pytest.mark.parametrize("n", [16, 17])
+@pytest.mark.parametrize("prec,tol", [("D", 1e-13), ("F", 5e-6)])
+def test_force_of_more_solutions_than_one_pass_takes(gpu, n, prec, tol):
+    """One pass over the gradient sums up to 16 solutions; the 17th adds to the
+    stored gradient.  On the smallest lattice (half a block of sites per
+    parity), against the sum of single-solution gradients: n roundings of
+    sums whose terms are at most n times the largest (n 2^-53 and n 2^-24)."""
+    dims = (4, 4, 4, 4)
+    lib = gpu.use(dims)
+    L = lib.create_L(prec, fields(dims))
+    xs = [lib.create_V(prec, synthetic.gaussian_source(dims, seed=50 + k, parity="odd"), "odd") for k in range(n)]
+    coef = [(-1) ** k * (0.5 + 0.125 * k) for k in range(n)]
+    got = lib.force(prec, L, xs, coef, "odd")
+    want = [np.zeros(g.shape) for g in got]
+    for c, x in zip(coef, xs):
+        for w, g in zip(want, lib.force(prec, L, [x], [1.0], "odd")):
+            w += c * g.astype(np.float64)
+    for x in xs:
+        lib.destroy_V(prec, x)
+    lib.destroy_L(prec, L)
+    for g, w in zip(got, want):
+        assert np.abs(g - w).max() <= tol * np.abs(w).max()
