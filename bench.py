@@ -455,8 +455,10 @@ def run_gpu(args):
         "target_32x32x32x64": target,
         "config4_batch": batch,
     }
-    # our kernel launches per step: 4 per iteration + restart/reliable-update kernels
-    line["gpu_launches"] = int(np.median(iters)) * 4 + 8 * int(np.median(rus)) + 8
+    # our kernel launches per step: one resident loop per reliable update, the
+    # update's own kernels (sum, two Dslashes, residual, copy, direction) and the
+    # start's (norm, two Dslashes, residual, two copies)
+    line["gpu_launches"] = 7 * int(np.median(rus)) + 6
     print(json.dumps(line))
     if pg is not None:
         pg.destroy_process_group()
