@@ -1066,6 +1066,12 @@ bool solver_loop_run(Prec pv, const LoopRun &q, const Launch &L)
     // faster one or equal up to 32^3x64 (FP64 844 / 824, FP32 429 / 412,
     // 12-real 394.5 / 394.3).
     if (ls.prec == Prec::Half && L.g->vh > kLoopMaxSites16) return false;
+    // Updating every shift's two vectors is a stream of its own, which the
+    // kernel's full occupancy moves faster than the loop's one block per SM:
+    // FP64, 12 shifts, 24^3x48 (0.33 M sites) 400.7 against 422.6 us per
+    // iteration, 20^3x40 (0.16 M) 227.0 against 215.3; FP32 218.1 against 208.9
+    // at 24^3x48.
+    if (q.mode == kLoopMs && L.g->vh > (pv == Prec::Double ? 200000 : 400000)) return false;
     if (pv == Prec::Double && ls.prec == Prec::Double) {
         if (q.mode == kLoopCg) return launch<double, double, kLoopCg>(q, L);
         if (q.mode == kLoopMs) return launch<double, double, kLoopMs>(q, L);
