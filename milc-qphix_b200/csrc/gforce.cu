@@ -32,10 +32,8 @@
 // multiplication (gf_program): 134 products of 3x3 matrices and 182 link
 // loads per link instead of 181 and 229.  The links come from L1/L2 (every
 // link is read by ~150 threads).  FP64 for D3, FP32 for F3.
-#include <algorithm>
 #include <cstring>
 #include <type_traits>
-#include <vector>
 
 #include "context.h"
 #include "device_common.cuh"
@@ -59,7 +57,7 @@ enum GfOp : unsigned { kStart = 0, kMul = 1, kMix = 2, kFold = 3 };
 // bits: 0-1 op, 2-3 axis of U, 4 adjoint, 5-7 add, 8 parity of the
 // displacement, 9 + 3a .. 11 + 3a displacement along a plus 2
 struct GfEntry {
-    static unsigned make(GfOp op, int axis, bool adj, int add, const int disp[4])
+    static constexpr unsigned make(GfOp op, int axis, bool adj, int add, const int disp[4])
     {
         unsigned e = (unsigned)op | (unsigned)axis << 2 | (unsigned)adj << 4 | (unsigned)add << 5;
         e |= (unsigned)((disp[0] + disp[1] + disp[2] + disp[3]) & 1) << 8;
@@ -68,14 +66,17 @@ struct GfEntry {
     }
 };
 constexpr int kGfProgram = 184;  // entries of the longest program
-// programs by which coefficients are non-zero (bit t: c_t) and direction
-__constant__ unsigned c_gf_program[8][4][kGfProgram];
-__constant__ int c_gf_length[8][4];
+// by which coefficients are non-zero (bit t: c_t) and direction
+struct GfPrograms {
+    unsigned entry[8][4][kGfProgram];
+    int length[8][4];
+};
 
-// The program of direction mu; terms with a zero coefficient are left out.
-std::vector<unsigned> gf_program(int mask, int mu)
+// Appends the program of direction mu to p; terms with a zero coefficient are
+// left out.  (Evaluated by the compiler; a program longer than kGfProgram
+// does not compile.)
+constexpr void gf_program(GfPrograms &p, int mask, int mu)
 {
-    std::vector<unsigned> p;
     const bool c0 = mask & 1, c1 = mask & 2, c2 = mask & 4;
     int pos[4] = {0, 0, 0, 0};
     // one step of a path from the current position (kStart and kMix: from x + mu)
@@ -83,17 +84,17 @@ std::vector<unsigned> gf_program(int mask, int mu)
         if (op == kStart || op == kMix)
             for (int d = 0; d < 4; ++d) pos[d] = d == mu;
         if (sign < 0) --pos[axis];
-        p.push_back(GfEntry::make(op, axis, sign < 0, coef, pos));
+        p.entry[mask][mu][p.length[mask][mu]++] = GfEntry::make(op, axis, sign < 0, coef, pos);
         if (sign > 0) ++pos[axis];
     };
-    if (!mask) return p;
+    if (!mask) return;
     for (int rho = 0; rho < 4; ++rho) {
         if (rho == mu) continue;
-        for (int r : {1, -1}) {
+        for (int r = 1; r >= -1; r -= 2) {
             if (c2)
                 for (int nu = 0; nu < 4; ++nu) {
                     if (nu == mu || nu == rho) continue;
-                    for (int s : {1, -1}) {  // parallelogram [nu s, rho r, -mu, -nu s, -rho r]
+                    for (int s = 1; s >= -1; s -= 2) {  // parallelogram [nu s, rho r, -mu, -nu s, -rho r]
                         add(kStart, nu, s);
                         add(kMul, rho, r);
                         add(kMul, mu, -1);
@@ -127,7 +128,7 @@ std::vector<unsigned> gf_program(int mask, int mu)
     if (c1) {  // rectangles [nu s, -mu, -mu, -nu s, mu]
         for (int nu = 0; nu < 4; ++nu) {
             if (nu == mu) continue;
-            for (int s : {1, -1}) {
+            for (int s = 1; s >= -1; s -= 2) {
                 add(kStart, nu, s);
                 add(kMul, mu, -1);
                 add(kMul, mu, -1);
@@ -136,8 +137,22 @@ std::vector<unsigned> gf_program(int mask, int mu)
         }
         add(kFold, mu, 1);
     }
+}
+
+constexpr GfPrograms gf_programs()
+{
+    GfPrograms p{};
+    for (int mask = 0; mask < 8; ++mask)
+        for (int mu = 0; mu < 4; ++mu) gf_program(p, mask, mu);
     return p;
 }
+
+// Part of the module's image, so that it is there whenever the kernel is.  (A
+// copy to a symbol at the first call runs on the default stream, which the
+// library's non-blocking stream does not wait for: a kernel that reads the
+// length before it lands adds no staple at all.)
+constexpr GfPrograms kGfPrograms = gf_programs();
+__constant__ GfPrograms c_gf = kGfPrograms;
 
 // One row of a product of 3x3 complex matrices (row-major reals u[6 r + 2 c] +
 // i u[6 r + 2 c + 1]): t = (a_0, a_1, a_2) b or b^dag, as chains of fused
@@ -290,8 +305,8 @@ k_gauge_force(GaugeView<R> U, cx_t<R> *mom, int cb, R eps, R c0, R c1, R c2, int
         if constexpr (kGfSharedX<R>) sh.x[i][tid] = R(0);
         else X[i] = R(0);
     }
-    const unsigned *prog = c_gf_program[mask][mu];
-    const int n = c_gf_length[mask][mu];
+    const unsigned *prog = c_gf.entry[mask][mu];
+    const int n = c_gf.length[mask][mu];
     auto apply = [&](unsigned e, const R u[18]) {
         if (e & 16u) gf_apply<true>(sh, e & 3u, u, M, X, c0, c1);
         else gf_apply<false>(sh, e & 3u, u, M, X, c0, c1);
@@ -554,27 +569,6 @@ void destroy(H *h)
     delete h;
 }
 
-bool g_table_ready[64] = {false};
-
-void upload_table()
-{
-    int dev = 0;
-    QB_CUDA(cudaGetDevice(&dev));
-    if (dev >= 0 && dev < 64 && g_table_ready[dev]) return;
-    static unsigned prog[8][4][kGfProgram];
-    int len[8][4];
-    for (int mask = 0; mask < 8; ++mask)
-        for (int mu = 0; mu < 4; ++mu) {
-            const std::vector<unsigned> p = gf_program(mask, mu);
-            if ((int)p.size() > kGfProgram) throw Error("gauge force: program too long");
-            len[mask][mu] = (int)p.size();
-            std::copy(p.begin(), p.end(), prog[mask][mu]);
-        }
-    QB_CUDA(cudaMemcpyToSymbol(c_gf_program, prog, sizeof(prog)));
-    QB_CUDA(cudaMemcpyToSymbol(c_gf_length, len, sizeof(len)));
-    if (dev >= 0 && dev < 64) g_table_ready[dev] = true;
-}
-
 // flops of one link's force, loop by loop: 2 (plaquette) or 4 (six-link
 // loops) 3x3 complex products per staple (198 flops each), its weighted sum
 // (36), U times the sum (198), TA and the update (54)
@@ -599,7 +593,6 @@ void gauge_force(QPHIX_info_t *info, typename GfApi<R>::G *G, typename GfApi<R>:
         require(F->parity == G->parity, "symanzik_1loop_gauge_force: force and gauge field parities differ");
         check_single_rank("symanzik_1loop_gauge_force");
         info->final_sec = wall_seconds();
-        upload_table();
         const int cb = G->parity == QPHIX_EVEN ? 0 : 1;
         GaugeView<R> U;
         U.b[0] = static_cast<const cx_t<R> *>(G->blk[0]);

@@ -148,3 +148,40 @@ def test_gauge_force_of_every_subset_of_loops(gpu, dims, which):
         assert np.abs(got - want).max() < 1e-12 * np.abs(want).max()
         lib.destroy_F("D", f)
         lib.destroy_G("D", g)
+
+
+FIRST_CALL = r"""
+import sys
+sys.path[:0] = [ROOT, ROOT + "/oracle"]
+import numpy as np
+import __graft_entry__ as e
+e.load_package()
+from milc_qphix_b200 import LIB_PATH, capi, synthetic
+import gauge_force_oracle as G
+dims, co = (4, 8, 4, 12), COEFFS
+lat = synthetic.Lattice(dims)
+U, A = G.random_su3_lex(dims, 7, 0.5), G.random_algebra_lex(dims, 8)
+want = G.momentum_update(U, A, co, 0.0375, G.parity_mask(dims, "even"))
+lib = capi.QphixLib(LIB_PATH)
+assert lib.init(dims) == 0, lib.last_error()
+g = lib.create_G("D", synthetic._to_raw_links(lat, U))
+f = lib.create_F("D", synthetic._to_raw_links(lat, A))
+assert lib.gauge_force("D", g, f, co, 0.0375).status == 0, lib.last_error()
+got = synthetic.links_raw_to_lex(dims, lib.extract_F("D", f))
+lib.destroy_F("D", f)
+lib.destroy_G("D", g)
+lib.finalize()
+assert np.abs(got - want).max() <= 1e-12 * np.abs(want).max(), np.abs(got - want).max()
+"""
+
+
+def test_first_gauge_force_of_a_process(gpu):
+    """The kernel's tables are there at the first call of a process."""
+    import os
+    import subprocess
+    import sys
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    code = f"ROOT = {root!r}\nCOEFFS = {COEFFS!r}\n" + FIRST_CALL
+    p = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0, p.stderr[-2000:]
