@@ -101,13 +101,13 @@ void init_context(QPHIX_layout_t *layout)
     c.g = make_geom(L[0], L[1], L[2], L[3]);
     halo_setup(c, P, comm_rank(), 2LL * c.g.vh * P);
     QB_CUDA(cudaMalloc(&c.d_state, sizeof(SolverState)));
-    QB_CUDA(cudaMemset(c.d_state, 0, sizeof(SolverState)));
+    QB_CUDA(cudaMemsetAsync(c.d_state, 0, sizeof(SolverState), c.stream));
     QB_CUDA(cudaMallocHost(&c.h_state, sizeof(SolverState)));
     std::memset(c.h_state, 0, sizeof(SolverState));
     QB_CUDA(cudaMalloc(&c.d_partials, sizeof(double) * 4 * kMaxPartials));
     QB_CUDA(cudaMalloc(&c.d_scalars, sizeof(double) * 64));
     QB_CUDA(cudaMalloc(&c.d_err, sizeof(int)));
-    QB_CUDA(cudaMemset(c.d_err, 0, sizeof(int)));
+    QB_CUDA(cudaMemsetAsync(c.d_err, 0, sizeof(int), c.stream));
     QB_CUDA(cudaMalloc(&c.d_slots, solver_loop_slot_bytes()));
     QB_CUDA(cudaMallocHost(&c.h_scalars, sizeof(double) * 64));
     for (int i = 0; i < 2; ++i) {

@@ -265,7 +265,7 @@ void sync_check()
     int e = 0;
     QB_CUDA(cudaMemcpy(&e, c.d_err, sizeof(int), cudaMemcpyDeviceToHost));
     if (e) {
-        QB_CUDA(cudaMemset(c.d_err, 0, sizeof(int)));
+        QB_CUDA(cudaMemsetAsync(c.d_err, 0, sizeof(int), c.stream));
         throw Error("a Dslash pipeline wait timed out on the GPU; the call's results are invalid");
     }
 }

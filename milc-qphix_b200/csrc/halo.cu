@@ -83,7 +83,7 @@ void halo_setup(Context &c, int nranks, int rank, long long global_sites)
         h.face_bytes[p] = (size_t)3 * c.g.st * site_bytes(p);
         char *g = nullptr;
         QB_CUDA(cudaMalloc(&g, 2 * h.face_bytes[p]));
-        QB_CUDA(cudaMemset(g, 0, 2 * h.face_bytes[p]));
+        QB_CUDA(cudaMemsetAsync(g, 0, 2 * h.face_bytes[p], c.stream));
         h.gback[p] = g;
         h.gfwd[p] = g + h.face_bytes[p];
         if (nranks > 1) {

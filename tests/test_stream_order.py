@@ -15,7 +15,7 @@ from conftest import ROOT
 
 CSRC = sorted(glob.glob(os.path.join(ROOT, "milc-qphix_b200", "csrc", "*")))
 # writes to device memory on the default stream
-DEFAULT_STREAM = re.compile(r"\bcudaMemcpyToSymbol\s*\(|\bcudaMemcpy\s*\([^;]*HostToDevice", re.S)
+DEFAULT_STREAM = re.compile(r"\bcudaMemset\s*\(|\bcudaMemcpyToSymbol\s*\(|\bcudaMemcpy\s*\([^;]*HostToDevice", re.S)
 
 
 @pytest.mark.parametrize("path", CSRC, ids=os.path.basename)
