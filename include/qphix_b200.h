@@ -130,12 +130,14 @@ int QPHIX_B200_tuning(int kernel, int p, double *us, int n);
  * which sets the value at load. */
 QPHIX_status_t QPHIX_B200_set_dslash_variant(int variant);
 
-/* Poll limit of the bounded mbarrier waits of the TMA-pipeline Dslash
- * (variant 2).  A wait that reaches the limit stops the kernel, which lets
- * the copies it issued land, records the failure in a device error word and
+/* Poll limit of the bounded waits: the mbarrier waits of the TMA Dslash
+ * kernels (variants 2 and 3) and the grid barriers of the resident solver
+ * loop.  A wait that reaches the limit stops the kernel, which lets the
+ * copies it issued land, records the failure in a device error word and
  * returns; the call then reports QPHIX_FAIL and QPHIX_B200_last_error says
- * so.  polls < 0 restores the default (2^22 polls, far longer than any copy
- * takes); 0 gives up at the first wait, which exercises the failure path. */
+ * which wait it was.  polls < 0 restores the default (2^22 polls, far longer
+ * than any copy or phase takes); 0 gives up at the first wait, which
+ * exercises the failure path. */
 QPHIX_status_t QPHIX_B200_set_wait_limit(long polls);
 
 /* ---- Operators of the inner solves (no counterpart in the reference) ------

@@ -266,7 +266,8 @@ void sync_check()
     QB_CUDA(cudaMemcpy(&e, c.d_err, sizeof(int), cudaMemcpyDeviceToHost));
     if (e) {
         QB_CUDA(cudaMemsetAsync(c.d_err, 0, sizeof(int), c.stream));
-        throw Error("a Dslash pipeline wait timed out on the GPU; the call's results are invalid");
+        throw Error(std::string(e == kErrLoopWait ? "a grid barrier of the solver loop" : "a Dslash pipeline wait") +
+                    " timed out on the GPU; the call's results are invalid");
     }
 }
 

@@ -356,7 +356,7 @@ template <> struct TmaCfg<__half> { static constexpr int C = 9, T = 128, NS = 4;
 
 constexpr unsigned kDefaultWaitPolls = 1u << 22;  // far longer than any copy takes
 constexpr unsigned kDrainPolls = 1u << 22;
-// poll limit of the pipeline's waits (QPHIX_B200_set_wait_limit)
+// poll limit of the bounded waits (QPHIX_B200_set_wait_limit)
 static unsigned g_wait_limit = kDefaultWaitPolls;
 
 template <typename S>
@@ -510,7 +510,7 @@ k_dslash_tma(DslashArgs<SV, SL> a, const char *links, VecView<SV> pv, double m4,
     }
     if (failed) {
         if (tid == 0) {
-            atomicExch(err, 1);
+            atomicExch(err, kErrDslashWait);
             // stages g .. g+NS-1 may still be in flight, one per barrier
             const int last = min(g + NS - 1, total - 1);
             for (int s2 = g; s2 <= last; ++s2)
@@ -620,7 +620,7 @@ k_dslash_tile(DslashArgs<SV, SL> a, VecView<SV> pv, double m4, SolverState *st, 
     }
     if (failed) {
         if (tid == 0) {
-            atomicExch(err, 1);
+            atomicExch(err, kErrDslashWait);
             // the plane's copies may still be in flight (the phase just waited on)
             (void)mbar_wait_bounded(bar, phase ^ 1u, kDrainPolls);
         }
@@ -718,6 +718,8 @@ void set_wait_limit(long polls)
 {
     g_wait_limit = polls < 0 ? kDefaultWaitPolls : (unsigned)std::min<long>(polls, 0x7fffffffL);
 }
+
+unsigned wait_limit() { return g_wait_limit; }
 
 struct TuneEntry {
     int vh = -1;

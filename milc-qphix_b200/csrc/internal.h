@@ -210,8 +210,15 @@ int dslash_variant(int kernel, Prec pv, int slot, float us[4]);
 constexpr int kDslashVariants = 4;
 // -1: autotuned variants; 0..2: that variant everywhere
 void set_forced_variant(int v);
-// poll limit of the TMA pipeline's waits (< 0: the default)
+// poll limit of the TMA pipelines' waits and the solver loop's grid barriers
+// (< 0: the default)
 void set_wait_limit(long polls);
+unsigned wait_limit();
+// values of the failure word
+enum : int {
+    kErrDslashWait = 1,  // a copy of a pipelined Dslash did not land
+    kErrLoopWait = 2,    // a grid barrier of the resident solver loop
+};
 
 // BLAS (blas.cu) ---------------------------------------------------------------
 // state->source_norm = |v|^2

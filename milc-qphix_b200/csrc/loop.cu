@@ -21,8 +21,9 @@
 // with a sum (every block reads all partials).  Publishing {value, epoch}
 // words per block and polling all of them, without atomics, took 6.5 k: 148
 // blocks polling 148 words load the L2 more than one hot word does.  Every
-// wait is bounded; a wait that runs out stores the failure word and the block
-// returns.
+// wait is bounded (wait_limit() polls); a block whose wait runs out stores the
+// failure word and returns, and so do the others, whose next wait then cannot
+// end.
 //
 // Dslash: a group of PARTS * SG threads owns SG consecutive sites; part k of
 // the group (SG threads) applies one direction's links of one hop (8 parts) or
@@ -55,7 +56,6 @@ namespace qb {
 namespace {
 
 constexpr int kLoopMaxBlocks = 256;         // partial sums per buffer
-constexpr unsigned kLoopPolls = 1u << 22;   // poll limit of a barrier wait
 
 // most threads of a block: 64 registers each for FP32 sums, 128 for FP64
 // eight_parts: largest lattice (sites per parity) whose Dslash is split into
@@ -92,6 +92,7 @@ struct LoopArgs {
     unsigned *counter;      // barrier arrivals
     double *partials;       // [2 parities of the epoch][block]
     int *err;
+    unsigned polls;         // poll limit of a barrier wait
     int sg, lg_sg;          // sites of a group (4..32) and its logarithm
     int groups;             // groups of a block
     FastDiv dx, dy, dz;     // by Nxh, Ny, Nz
@@ -123,6 +124,7 @@ struct LoopShared {
 struct LoopBarrier {
     unsigned *counter;
     double *partials;
+    unsigned polls;
     unsigned epoch;
 };
 
@@ -136,8 +138,8 @@ __device__ __forceinline__ bool grid_wait(LoopShared &sh, LoopBarrier &b)
         arrive_release(b.counter);
         const unsigned target = b.epoch * gridDim.x;  // modulo 2^32, as the counter
         unsigned k = 0;
-        while ((int)(load_acquire(b.counter) - target) < 0 && k < kLoopPolls) ++k;
-        if (k >= kLoopPolls) sh.fail = 1;
+        while (k < b.polls && (int)(load_acquire(b.counter) - target) < 0) ++k;
+        if (k >= b.polls) sh.fail = 1;
     }
     __syncthreads();
     return sh.fail == 0;
@@ -697,7 +699,7 @@ __global__ void __launch_bounds__(LoopThreads<SV>::value, 1) k_solver_loop(const
     const int vh = a.g.vh, par = a.parity;
     const bool warp0 = threadIdx.x < 32;
     constexpr bool kMs = MODE == kLoopMs || MODE == kLoopMsDefer;
-    LoopBarrier bar{a.counter, a.partials, 0};
+    LoopBarrier bar{a.counter, a.partials, a.polls, 0};
     const GroupPlace place = group_place<PARTS>(a);
     bool ok = true;
     for (;;) {
@@ -778,7 +780,7 @@ __global__ void __launch_bounds__(LoopThreads<SV>::value, 1) k_solver_loop(const
         if (!(ok = grid_wait(sh, bar))) break;
     }
     if (!ok) {
-        if (threadIdx.x == 0) atomicExch(a.err, 1);
+        if (threadIdx.x == 0) atomicExch(a.err, kErrLoopWait);
         return;
     }
     if (blockIdx.x == 0) {
@@ -817,7 +819,7 @@ __global__ void __launch_bounds__(SmallThreads<SV>::value, 1) k_small_loop(const
     const int vh = a.g.vh, par = a.parity;
     const bool warp0 = threadIdx.x < 32;
     constexpr bool kMs = MODE == kLoopMsDefer;
-    LoopBarrier bar{a.counter, a.partials, 0};
+    LoopBarrier bar{a.counter, a.partials, a.polls, 0};
     const GroupPlace place = group_place<8>(a);
     const int n = 6 * vh / F::n, flat0 = blockIdx.x * blockDim.x + threadIdx.x, flat_step = gridDim.x * blockDim.x;
     VecView<SV> cur = a.p, other = a.p2;
@@ -893,7 +895,7 @@ __global__ void __launch_bounds__(SmallThreads<SV>::value, 1) k_small_loop(const
         if (S.stop_at != INT_MAX) break;
     }
     if (!ok) {
-        if (threadIdx.x == 0) atomicExch(a.err, 1);
+        if (threadIdx.x == 0) atomicExch(a.err, kErrLoopWait);
         return;
     }
     // the direction as the four-phase loop leaves it, in the caller's buffer
@@ -1012,6 +1014,7 @@ bool launch(const LoopRun &q, const Launch &L)
     a.counter = static_cast<unsigned *>(q.slots);
     a.partials = static_cast<double *>(q.slots) + 4;
     a.err = L.err;
+    a.polls = wait_limit();
     a.n = q.n;
     a.xs = q.xs;
     a.ps = q.ps;

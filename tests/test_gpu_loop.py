@@ -92,3 +92,30 @@ def test_backward_links_that_are_not_shifted_forward_links(gpu, monkeypatch, mod
     assert rel_err(x[0], x0[0]) < MODES[mode]
     _, y = _solve(lib, mode, links, src, "even", 6, [0.3])
     assert rel_err(y[0], x0[0]) > 30 * MODES["single" if mode != "double" else "double"]
+
+
+@pytest.mark.parametrize("mode,kernel", [("double", "k_solver_loop"), ("F", "k_solver_loop"), ("r12", "k_small_loop")])
+def test_barrier_wait_that_runs_out(gpu, mode, kernel):
+    """A poll limit of zero ends the first grid barrier: every block stores the
+    failure word and returns, and the call reports it.  A multi-shift solve
+    launches no other kernel with bounded waits before its loop (FP64 and FP32
+    shifts run in k_solver_loop, the deferred ones of a small lattice in
+    k_small_loop).  The next solve is the one without a failure, bit for
+    bit."""
+    dims = (8, 8, 8, 8)
+    lib = gpu.use(dims)
+    src = synthetic.gaussian_source(dims, seed=8, parity="even")
+    args = (lib, mode, fields(dims), src, "even", 10, [0.5, 0.3, 0.4])
+    want = _solve(*args)
+    try:
+        assert lib.set_wait_limit(0) == 0
+        with pytest.raises(AssertionError, match="grid barrier of the solver loop timed out"):
+            _solve(*args)
+        with pytest.raises(AssertionError, match="timed out"):  # (a tuned Dslash may be the first to wait)
+            _solve(lib, mode, fields(dims), src, "even", 10, [0.3])
+    finally:
+        lib.set_wait_limit(-1)
+    got = _solve(*args)
+    assert got[0] == want[0]
+    for a, b in zip(got[1], want[1]):
+        assert np.array_equal(a, b)
