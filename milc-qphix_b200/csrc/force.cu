@@ -110,6 +110,23 @@ template <> struct ForceApi<float> {
     static constexpr Prec prec = Prec::Single;
 };
 
+// Adds up to `extra` vectors to y, within half of the memory that is left, and
+// returns how many: a call that has room for one vector only takes passes of
+// one solution.  (Called after the first Dslash, whose tuning needs scratch of
+// its own.)
+static int more_vecs(std::vector<VecBlock> &y, int extra, Prec p)
+{
+    const size_t bytes = vec_bytes(p, ctx().g.vh);
+    extra = (int)std::min<size_t>(extra, extra > 0 ? dev_available() / 2 / bytes : 0);
+    for (int k = 0; k < extra; ++k) {
+        VecBlock v;
+        v.data = dev_try_alloc(bytes);
+        if (!v.data) return k;
+        y.push_back(v);
+    }
+    return extra;
+}
+
 template <typename Real>
 static void force_impl(typename ForceApi<Real>::FL *H, int n, const Real *coef, typename ForceApi<Real>::CV **x,
                        QPHIX_evenodd_t parity, Real *grad_fat, Real *grad_lng)
@@ -129,18 +146,20 @@ static void force_impl(typename ForceApi<Real>::FL *H, int n, const Real *coef, 
     Real *g = static_cast<Real *>(dev_alloc(2 * nraw * sizeof(Real)));
     std::vector<VecBlock> y;
     try {
-        for (int k = 0; k < std::min(n, kForceMax); ++k) y.push_back(alloc_vec(ForceApi<Real>::prec));
+        y.push_back(alloc_vec(ForceApi<Real>::prec));
         QB_CUDA(cudaEventRecord(c.ev_solve[0], c.stream));
         const int grid = (int)((8LL * c.g.vh + kBlock - 1) / kBlock);
-        for (int k0 = 0; k0 < n; k0 += kForceMax) {
+        int group = 1;  // solutions of one pass
+        for (int k0 = 0; k0 < n; k0 += group) {
             ForceIn<Real> f;
-            f.n = std::min(n - k0, kForceMax);
-            for (int k = 0; k < f.n; ++k) {
+            for (int k = 0; k < group && k0 + k < n; ++k) {
                 const VecBlock xb = x[k0 + k]->blk[P];
                 dslash(ForceApi<Real>::prec, L, y[k], xb, H->links, 1 - P);  // y = D_qp x
+                if (k0 == 0 && k == 0) group += more_vecs(y, std::min(n, kForceMax) - 1, ForceApi<Real>::prec);
                 f.x[k] = view<Real>(xb, c.g.vh);
                 f.y[k] = view<Real>(y[k], c.g.vh);
                 f.coef[k] = coef[k0 + k];
+                f.n = k + 1;
             }
             if (k0 == 0) k_force<Real, false><<<grid, kBlock, 0, c.stream>>>(g, g + nraw, f, c.g, P);
             else k_force<Real, true><<<grid, kBlock, 0, c.stream>>>(g, g + nraw, f, c.g, P);

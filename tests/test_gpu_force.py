@@ -192,3 +192,60 @@ def test_force_of_more_solutions_than_one_pass_takes(gpu, n, prec, tol):
     lib.destroy_L(prec, L)
     for g, w in zip(got, want):
         assert np.abs(g - w).max() <= tol * np.abs(w).max()
+
+
+LITTLE_MEMORY = r"""
+import sys
+sys.path.insert(0, ROOT)
+import numpy as np
+import torch
+import __graft_entry__ as e
+e.load_package()
+from milc_qphix_b200 import LIB_PATH, capi
+dims, n = (24, 24, 24, 24), 16
+V = int(np.prod(dims))
+nbytes = 24 * V  # one parity of an FP64 vector
+rng = np.random.default_rng(5)
+lib = capi.QphixLib(LIB_PATH)
+assert lib.init(dims) == 0, lib.last_error()
+a = rng.standard_normal(72 * V)
+L = lib.create_L("D", {k: a for k in ("fat", "lng", "fatback", "lngback")})
+xs = [lib.create_V("D", rng.standard_normal(6 * V), "even") for _ in range(n)]
+coef = [0.5 + 0.125 * k for k in range(n)]
+# the first calls leave the gradient's memory and one vector's with the library
+want = [0.0, 0.0]
+for x, c in zip(xs, coef):
+    g = lib.force("D", L, [x], [c], "even")
+    want = [w + q for w, q in zip(want, g)]
+hog = []
+while torch.cuda.mem_get_info()[0] > 6 * nbytes + (4 << 20):
+    hog.append(torch.empty(torch.cuda.mem_get_info()[0] - 6 * nbytes - (2 << 20), dtype=torch.uint8, device="cuda"))
+print("left", torch.cuda.mem_get_info()[0] / nbytes)
+got = lib.force("D", L, xs, coef, "even")
+del hog
+torch.cuda.empty_cache()
+for g, w in zip(got, want):
+    err = np.abs(g - w).max() / np.abs(w).max()
+    print(err)
+    assert err <= 1e-14, err
+lib.finalize()
+"""
+
+
+def test_force_with_little_memory_left():
+    """With room for a few of the scratch vectors D x only, the solutions are
+    summed in smaller groups and the call succeeds, as one pass per solution
+    would.  In a process of its own, whose library holds no memory of other
+    tests; of the GPU's memory all but six vectors' bytes are taken.  The
+    gradient differs by the order of a sum of n = 16 terms of either
+    sign, of which none is above the largest gradient entry by more than a few:
+    16 roundings of 2^-53 each, 1.8e-15, times that few."""
+    import os
+    import subprocess
+    import sys
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    p = subprocess.run([sys.executable, "-c", f"ROOT = {root!r}\n" + LITTLE_MEMORY], capture_output=True, text=True,
+                       timeout=300)
+    assert p.returncode == 0, p.stdout + p.stderr[-2000:]
+    print(p.stdout)
