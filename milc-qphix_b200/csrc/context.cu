@@ -41,18 +41,6 @@ void *dev_try_alloc(size_t bytes)
     return p;
 }
 
-size_t dev_available()
-{
-    size_t free_b = 0, total_b = 0;
-    QB_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    cudaMemPool_t pool;
-    QB_CUDA(cudaDeviceGetDefaultMemPool(&pool, ctx().device));
-    uint64_t reserved = 0, used = 0;
-    QB_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved));
-    QB_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
-    return free_b + (size_t)(reserved - used);
-}
-
 void dev_free(void *p)
 {
     if (p) cudaFreeAsync(p, ctx().stream);

@@ -126,7 +126,6 @@ void halo_free(Context &c);
 // device memory from the stream-ordered pool (cached, no device-wide sync)
 void *dev_alloc(size_t bytes);
 void *dev_try_alloc(size_t bytes);  // nullptr where the memory does not suffice
-size_t dev_available();             // bytes not in use: free on the device or kept by the pool
 void dev_free(void *p);
 
 // Host -> device copy that has completed on return.  Pinned or small
