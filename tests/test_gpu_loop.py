@@ -14,6 +14,7 @@ import numpy as np
 import pytest
 
 from conftest import fields, rel_err, synthetic
+from fixedpoint import naik_phased
 
 pytestmark = pytest.mark.gpu
 
@@ -25,8 +26,8 @@ MODES = {"double": 1e-12, "F": 1e-4, "single": 1e-4, "r12": 1e-4, "half-links": 
 
 def _solve(lib, mode, links, src, parity, n, masses):
     prec = "F" if mode == "F" else "D"
-    lib.set_inner_precision({"F": "double", "r12": "single"}.get(mode, mode))
-    lib.set_link_compression(mode == "r12")
+    lib.set_inner_precision({"F": "double", "r12": "single", "r13": "single"}.get(mode, mode))
+    lib.set_link_compression(mode in ("r12", "r13"))
     try:
         L = lib.create_L(prec, links)
         b = lib.create_V(prec, src, parity)
@@ -119,3 +120,71 @@ def test_barrier_wait_that_runs_out(gpu, mode, kernel):
     assert got[0] == want[0]
     for a, b in zip(got[1], want[1]):
         assert np.array_equal(a, b)
+
+
+# 65536 sites per parity: 151 MB of 18-real, 126 MB of 12- and 13-real and
+# 75 MB of 16-bit links, all read once per site where they are mirrored
+LARGE = (16, 16, 16, 32)
+_large = {}
+
+
+def _large_links(mode):
+    if not _large:
+        _large["links"] = synthetic.asqtad_links(LARGE, seed=1001, device="cuda")
+    if mode == "r13" and "r13" not in _large:
+        _large["r13"] = naik_phased(LARGE, _large["links"])
+    return _large["r13" if mode == "r13" else "links"]
+
+
+RECON = {"single": 0, "r12": 1, "r13": 2, "half-links": 0, "half": 0}
+
+
+@pytest.mark.parametrize("changed", [None, "fatback", "lngback"])
+@pytest.mark.parametrize("mode", list(RECON))
+def test_mirrored_storages(gpu, monkeypatch, mode, changed):
+    """Every inner storage where its links are read in their own site's block:
+    the sign bits (12-real) and ratios (13-real) come from there too, and the
+    16-bit records are read at other offsets.  With one backward link changed
+    (a Naik link by its phase, which keeps it 13-real but not 12-real) the
+    caller's backward links must be read."""
+    lib = gpu.use(LARGE)
+    links = _large_links(mode)
+    recon = RECON[mode]
+    if changed:
+        links = dict(links, **{changed: links[changed].copy()})
+        z = links[changed][72 * 4321:72 * 4321 + 18].view(np.complex128)
+        z *= 1.5 if changed == "fatback" else np.exp(1.0j)
+        if changed == "lngback" and mode == "r12":
+            recon = 2
+    src = synthetic.gaussian_source(LARGE, seed=9, parity="odd")
+    (it, x), (it0, x0) = _both(lib, monkeypatch, mode, links, src, "odd", 8, [0.3])
+    assert lib.last_stats().links_compressed == recon
+    assert it == it0
+    tol = {"r13": 1e-4}.get(mode, MODES.get(mode))
+    assert rel_err(x[0], x0[0]) < tol
+
+
+@pytest.mark.parametrize("mode", ["single", "r12", "r13"])
+def test_mirrored_multishift(gpu, monkeypatch, mode):
+    """The deferred shifts' loop (kLoopMsDefer) on mirrored links."""
+    lib = gpu.use(LARGE)
+    src = synthetic.gaussian_source(LARGE, seed=10, parity="even")
+    (it, x), (it0, x0) = _both(lib, monkeypatch, mode, _large_links(mode), src, "even", 8, [0.5, 0.3, 0.4])
+    assert it == it0
+    for a, b in zip(x, x0):
+        assert rel_err(a, b) < 1e-4
+
+
+@pytest.mark.parametrize("mode", ["double", "F", "single", "r12", "r13", "half-links", "half"])
+@pytest.mark.parametrize("masses", [[0.3], [0.5, 0.3, 0.4]], ids=["cg", "multishift"])
+def test_eight_parts_in_four_phases(gpu, monkeypatch, mode, masses):
+    """12^4 (10368 sites per parity): too large for the three-phase loop, eight
+    parts a site, links that are not read as mirrored."""
+    dims = (12, 12, 12, 12)
+    lib = gpu.use(dims)
+    links = naik_phased(dims, fields(dims)) if mode == "r13" else fields(dims)
+    src = synthetic.gaussian_source(dims, seed=11, parity="even")
+    (it, x), (it0, x0) = _both(lib, monkeypatch, mode, links, src, "even", 8, masses)
+    assert it == it0
+    for a, b in zip(x, x0):
+        assert rel_err(a, b) < {"r13": 1e-4}.get(mode, MODES.get(mode))
