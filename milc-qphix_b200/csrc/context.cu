@@ -48,15 +48,22 @@ void dev_free(void *p)
 
 namespace {
 
-// One pinned slot, and the smallest copy that goes through the slots.  The
-// first slot's transfer and the last slot's host copy overlap nothing, so small
-// slots shorten both ends; with 1 MB the copies' own cost shows.  ms for
-// 191 MB device -> host / 32 MB device -> host / 1.5 GB host -> device, with
-// 8 workers and 8 MB slots 6.2 / 1.9 / 41, 8 and 2 MB 5.4 / 1.2 / 36, 12 and
-// 2 MB 4.9 / 1.2 / 35, 16 and 1 MB 4.8 / 1.3 / 43 (16 host cores).
+// One pinned slot.  The first slot's transfer and the last slot's host copy
+// overlap nothing, so small slots shorten both ends; with 1 MB the copies' own
+// cost shows.  ms for 191 MB device -> host / 32 MB device -> host / 1.5 GB
+// host -> device, with 8 workers and 8 MB slots 6.2 / 1.9 / 41, 8 and 2 MB
+// 5.4 / 1.2 / 36, 12 and 2 MB 4.9 / 1.2 / 35, 16 and 1 MB 4.8 / 1.3 / 43 (16
+// host cores).  Four processes on that host at once copy 2 x 15 MiB up in
+// 2.7-3.3 ms with 12 workers each, 1.2-2.5 with 8.
 constexpr size_t kStageBytes = 2u << 20;
-constexpr size_t kStageMinBytes = 4u << 20;
 constexpr unsigned kStageWorkers = 12;
+// The smallest copy that goes through the slots: starting and joining the
+// workers takes 0.15 ms, which pays from 9 MiB up and 12 MiB down.  ms of two
+// copies in one call / through the slots, up and down: 4.5 MiB 0.49 / 0.62
+// and 0.57 / 0.76, 7.5 MiB 0.74 / 0.80 and 0.88 / 0.98, 12 MiB 1.14 / 1.02
+// and 1.34 / 1.23, 15 MiB 1.40 / 1.17 and 1.66 / 1.28.  The first staged copy
+// after QPHIX_init also makes the slots and streams, 45-100 ms.
+constexpr size_t kStageMinBytes = 12u << 20;
 
 void make_staging(Context &c)
 {
