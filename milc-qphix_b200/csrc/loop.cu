@@ -917,13 +917,14 @@ void check(cudaError_t e, const char *what)
     if (e != cudaSuccess) throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(e));
 }
 
-// bytes of the links of both parities
-size_t loop_link_bytes(const LinkSet &ls, int vh)
-{
-    const size_t per_site = ls.recon ? (size_t)kReconChunks * 64 : ls.prec == Prec::Double ? 2304
-                                                                  : ls.prec == Prec::Single ? 1152 : 576;
-    return 2 * per_site * vh;
-}
+// bytes of the links of one site of a parity block
+template <typename SL> constexpr size_t kLinkBytes = 72 * sizeof(cx_t<SL>) * 2;
+template <> constexpr size_t kLinkBytes<__half> = 576;
+template <> constexpr size_t kLinkBytes<Recon12> = (size_t)kReconChunks * 64;
+template <> constexpr size_t kLinkBytes<Recon13> = (size_t)kReconChunks * 64;
+
+// the links of both parities that the loop reads as mirrored (loop_wants_mirrored)
+constexpr size_t kMirroredMin = (size_t)64 << 20, kMirroredMax = (size_t)152 << 20;
 
 constexpr int kLoopMaxSites16 = 500000;
 
@@ -1027,8 +1028,12 @@ bool launch(const LoopRun &q, const Launch &L)
         }
     }
     const bool eight = vh <= LoopThreads<SV>::eight_parts;
-    if (q.links->mirrored == 1 && loop_wants_mirrored(*q.links, vh))
-        return eight ? launch_form<SV, SL, MODE, true, 8>(a, L) : launch_form<SV, SL, MODE, true, 4>(a, L);
+    if (q.links->mirrored == 1 && loop_wants_mirrored(*q.links, vh)) {
+        // (only FP64 links are large enough for it on a lattice of eight parts)
+        if constexpr (2 * kLinkBytes<SL> * LoopThreads<SV>::eight_parts >= kMirroredMin)
+            if (eight) return launch_form<SV, SL, MODE, true, 8>(a, L);
+        return launch_form<SV, SL, MODE, true, 4>(a, L);
+    }
     return eight ? launch_form<SV, SL, MODE, false, 8>(a, L) : launch_form<SV, SL, MODE, false, 4>(a, L);
 }
 
@@ -1045,8 +1050,11 @@ size_t solver_loop_slot_bytes() { return (4 + 2 * kLoopMaxBlocks) * sizeof(doubl
 // 16-bit) 69.3 / 63.0; 302 MB (16^3x32 FP64) 60.4 / 60.9.
 bool loop_wants_mirrored(const LinkSet &ls, int vh)
 {
-    const size_t bytes = loop_link_bytes(ls, vh);
-    return bytes >= ((size_t)64 << 20) && bytes <= ((size_t)152 << 20);
+    const size_t site = ls.recon ? kLinkBytes<Recon12> : ls.prec == Prec::Double ? kLinkBytes<double>
+                                                      : ls.prec == Prec::Single ? kLinkBytes<float>
+                                                                                : kLinkBytes<__half>;
+    const size_t bytes = 2 * site * vh;
+    return bytes >= kMirroredMin && bytes <= kMirroredMax;
 }
 
 bool solver_loop_wants_p2(Prec pv, const Launch &L)
