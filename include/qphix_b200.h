@@ -79,8 +79,16 @@ typedef struct {
 
 QPHIX_status_t QPHIX_B200_get_last_stats(QPHIX_B200_stats_t *stats);
 
+/* Phases of the most recent invert / invert_multi call (a CG pass between
+ * restarts, a mixed-precision run between reliable updates, a multi-shift
+ * pass) that ran in the resident solver loop, one cooperative launch each; 0
+ * when all its phases ran as separate kernels (several GPUs, a forced Dslash
+ * variant, kernel timing, a relative residue, QPHIX_B200_LOOP=0, ...). */
+int QPHIX_B200_last_loop_launches(void);
+
 /* Per-launch CUDA-event timing of the Dslash kernels inside solves
- * (0 = off, the default). */
+ * (0 = off, the default).  Solves timed this way run the separate kernels,
+ * not the resident loop. */
 QPHIX_status_t QPHIX_B200_set_kernel_timing(int on);
 
 /* Device timer on the library's CUDA stream: start, then stop returns the

@@ -277,6 +277,10 @@ class QphixLib:
         self.lib.QPHIX_B200_get_last_stats(C.byref(s))
         return s
 
+    def last_loop_launches(self):
+        """Phases of the last solve that ran in the resident loop."""
+        return self.lib.QPHIX_B200_last_loop_launches()
+
     def set_kernel_timing(self, on):
         return self.lib.QPHIX_B200_set_kernel_timing(1 if on else 0)
 

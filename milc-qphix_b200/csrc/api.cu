@@ -828,6 +828,7 @@ QPHIX_status_t QPHIX_B200_get_last_stats(QPHIX_B200_stats_t *s)
         s->escalated = t.escalated;
     });
 }
+int QPHIX_B200_last_loop_launches(void) { return ctx().stats.loop_launches; }
 QPHIX_status_t QPHIX_B200_set_kernel_timing(int on) { return guarded([&] { ctx().kernel_timing = on ? 1 : 0; }); }
 QPHIX_status_t QPHIX_B200_timer_start(void)
 {

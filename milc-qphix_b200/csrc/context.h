@@ -49,6 +49,7 @@ struct Stats {
     int escalated = 0;
     int links_compressed = 0;
     int batch_rhs_per_thread = 0;
+    int loop_launches = 0;  // solver phases that ran in the resident loop
 };
 
 // CUDA-event timing of individual kernel launches inside a solve

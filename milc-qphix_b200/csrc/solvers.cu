@@ -175,6 +175,7 @@ public:
             S.err = nullptr;  // the loop reports a failed wait itself
             upload_state();
             if (solver_loop_run(pv, *res, c.launch())) {
+                ++c.stats.loop_launches;
                 download_state();
                 if (S.stop_at == INT_MAX) throw Error("solver: device loop ended without a stop");
                 return;

@@ -188,3 +188,31 @@ def test_eight_parts_in_four_phases(gpu, monkeypatch, mode, masses):
     assert it == it0
     for a, b in zip(x, x0):
         assert rel_err(a, b) < {"r13": 1e-4}.get(mode, MODES.get(mode))
+
+
+@pytest.mark.parametrize("mode", ["double", "F", "r12"])
+@pytest.mark.parametrize("masses", [[0.3], [0.5, 0.3, 0.4]], ids=["cg", "multishift"])
+def test_loop_launches_are_counted(gpu, monkeypatch, mode, masses):
+    """The count says which route a solve took: the loop, or the kernels with
+    the loop switched off, a forced Dslash variant or kernel timing."""
+    dims = (8, 8, 8, 8)
+    lib = gpu.use(dims)
+    src = synthetic.gaussian_source(dims, seed=12, parity="even")
+    args = (lib, mode, fields(dims), src, "even", 10, masses)
+    _solve(*args)
+    assert lib.last_loop_launches() >= 1
+    monkeypatch.setenv("QPHIX_B200_LOOP", "0")
+    _solve(*args)
+    assert lib.last_loop_launches() == 0
+    monkeypatch.delenv("QPHIX_B200_LOOP")
+    try:
+        lib.set_dslash_variant(1)
+        _solve(*args)
+        assert lib.last_loop_launches() == 0
+        lib.set_dslash_variant(-1)
+        lib.set_kernel_timing(True)
+        _solve(*args)
+        assert lib.last_loop_launches() == 0
+    finally:
+        lib.set_dslash_variant(-1)
+        lib.set_kernel_timing(False)
