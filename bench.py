@@ -53,6 +53,12 @@ DSLASH_BYTES_R12 = 1012  # FP32 with 12-real Naik links: 8x72 + 8x48 + 4 (sign w
 K1_TRAFFIC_PER_SITE_F32 = 264.33e6 / 221184
 # 332.36 MB (327.83 read + 4.53 write) at 24^3x48 for the pipelined k_dslash<float, Recon12>
 K1_TRAFFIC_PER_SITE_R12 = 332.361728e6 / 331776
+# vectors of an iteration besides the two Dslash applications: r (read and
+# written) and ttt, then x and p (read and written) and r
+VECTOR_BYTES_F32 = 72 + 120
+# DRAM bytes per output site and iteration of k_solver_loop<float, Recon12>
+# measured by ncu: 19.64 GB (19.138 read + 0.500 write) in 30 iterations at 24^3x48
+LOOP_TRAFFIC_PER_SITE_R12 = 19.638e9 / 30 / 331776
 DSLASH_FLOPS = 1146
 METRIC = "time to |r|/|b|<1e-10, mixed vs FP64 CG on 1 B200; Dslash HBM GB/s"
 VARIANTS = ["resident-grid", "full-grid", "tma-link-pipeline", "tma-neighbour-tiles"]
@@ -182,6 +188,15 @@ def max_over_ranks(pg, v):
     return float(t.item())
 
 
+def mixed_solve_launches(iterations, updates, loops):
+    """Kernel launches of one mixed CG solve.  Every reliable update: x += x_s,
+    two Dslashes and the residual, and (not after the last) the copy of r and
+    the direction; before the first run the norm, two Dslashes, the residual and
+    two copies.  The iterations: one launch per run in the resident loop, four
+    kernels each otherwise."""
+    return 4 + 6 * updates + (loops if loops else 4 * iterations)
+
+
 def make_inputs(device=None, dims=DIMS):
     # the eigendecompositions of the generator run on the host (torch CPU)
     # unless a device is given
@@ -237,7 +252,7 @@ def run_gpu(args):
     clocks = ClockSampler(local)
     barrier(pg)
     clocks.start()
-    times, iters, rus, trues = [], [], [], []
+    times, iters, rus, trues, loops, launches = [], [], [], [], [], 0
     xs_last = None
     for k in range(args.steps):
         x, ms, res, st = solve("single")
@@ -245,6 +260,8 @@ def run_gpu(args):
         iters.append(st.iterations)
         rus.append(st.reliable_updates)
         trues.append(res.final_rsq)
+        loops.append(lib.last_loop_launches())
+        launches += mixed_solve_launches(st.iterations, st.reliable_updates, loops[-1])
         if k == args.steps - 1:
             xs_last = lib.extract_V("D", x, "even")[: Vh * 6]
         lib.destroy_V("D", x)
@@ -252,8 +269,9 @@ def run_gpu(args):
     clk = clocks.stop()
     ms_step = max_over_ranks(pg, float(np.mean(times)))
 
-    # per-kernel CUDA-event durations from one more solve of the same input
-    # (events around every launch cost host time, so not inside the timed steps)
+    # per-kernel CUDA-event durations from one more solve of the same input with
+    # the separate kernels (the timed solves run the resident loop, which has no
+    # launches to put events around)
     lib.set_kernel_timing(True)
     x, ms_inst, _, st = solve("single")
     lib.destroy_V("D", x)
@@ -375,6 +393,12 @@ def run_gpu(args):
     k2_bytes = k1_bytes + 24
     k2_ms = mdagm_ms / max(mdagm_n, 1)
     k2_achieved = k2_bytes * Vh / (k2_ms * 1e-3) / 1e9
+    # the timed solves: time per iteration (reliable updates included) against
+    # the bytes of an iteration
+    it_bytes = k1_bytes + k2_bytes + VECTOR_BYTES_F32
+    it_us = ms_step * 1e3 / float(np.mean(iters))
+    it_achieved = it_bytes * Vh / (it_us * 1e-6) / 1e9
+    resident = min(loops) > 0
     err_vs_fp64 = float(np.abs(xs_last - xsol64).max() / np.abs(xsol64).max())
     err_half = float(np.abs(xsolh - xsol64).max() / np.abs(xsol64).max())
     err_hl = float(np.abs(xsoll - xsol64).max() / np.abs(xsol64).max())
@@ -424,19 +448,28 @@ def run_gpu(args):
                                      "us": [round(x, 2) for x in us]} for k, (v, us) in tuning.items()},
                    "autotuner_k2": {k: {"variant": VARIANTS[v] if v >= 0 else None,
                                         "us": [round(x, 2) for x in us]} for k, (v, us) in tuning_k2.items()}},
-        "roofline": {"kernel": ("k_dslash<float, Recon12>" if compressed else "k_dslash<float, float>")
-                               + " (K1) in a solve of the timed workload (CUDA events per launch)",
+        "roofline": {"kernel": ((("k_solver_loop<float, Recon12>" if compressed else "k_solver_loop<float, float>")
+                                 + ": the resident loop") if resident else "the separate kernels of an iteration")
+                               + " of the timed solves, per iteration, reliable updates included in the time",
                      "bound": "hbm",
-                     "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                     "peak_source": peak_kind, "algorithmic_bytes_per_site": k1_bytes,
-                     # ncu dram__bytes_read+write per output site of one K1 launch
+                     "achieved": it_achieved, "peak": peak, "unit": "GB/s", "frac": it_achieved / peak,
+                     "peak_source": peak_kind, "algorithmic_bytes_per_site": it_bytes,
+                     # ncu dram__bytes_read+write per output site and iteration
                      # (profiles/), times the sites of this lattice
-                     "traffic": (None if (compressed and K1_TRAFFIC_PER_SITE_R12 is None) else
-                                 (K1_TRAFFIC_PER_SITE_R12 if compressed else K1_TRAFFIC_PER_SITE_F32) * Vh),
-                     "launches": int(dslash_n), "avg_launch_us": k1_ms * 1e3},
+                     "traffic": LOOP_TRAFFIC_PER_SITE_R12 * Vh if compressed and resident else None,
+                     "loop_launches": int(np.median(loops)), "us_per_iteration": it_us},
+        "roofline_k1": {"kernel": ("k_dslash<float, Recon12>" if compressed else "k_dslash<float, float>")
+                                  + " (K1) in one more solve with the separate kernels, not in the timed steps (CUDA "
+                                    "events per launch)",
+                        "bound": "hbm",
+                        "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+                        "peak_source": peak_kind, "algorithmic_bytes_per_site": k1_bytes,
+                        # ncu dram__bytes_read+write per output site of one K1 launch
+                        "traffic": (K1_TRAFFIC_PER_SITE_R12 if compressed else K1_TRAFFIC_PER_SITE_F32) * Vh,
+                        "launches": int(dslash_n), "avg_launch_us": k1_ms * 1e3},
         "roofline_k2": {"kernel": ("k_dslash_mdagm<float, Recon12>" if compressed else "k_dslash_mdagm<float, float>")
-                                  + " (K2: Dslash + M^dag M epilogue + p.Mp reduction) in a solve of the timed "
-                                    "workload (CUDA events per launch)",
+                                  + " (K2: Dslash + M^dag M epilogue + p.Mp reduction) in the same solve with the "
+                                    "separate kernels",
                         "bound": "hbm", "achieved": k2_achieved, "peak": peak, "unit": "GB/s",
                         "frac": k2_achieved / peak, "peak_source": peak_kind,
                         "algorithmic_bytes_per_site": k2_bytes, "launches": int(mdagm_n),
@@ -449,16 +482,12 @@ def run_gpu(args):
         "e2e_links_resident": {"value": e2e_res_ms / 1e3, "unit": "s", "h2d_bytes_per_step": 2 * Vh * 6 * 8,
                                "d2h_bytes_per_step": Vh * 6 * 8, "steps": n_e2e,
                                "what": "as e2e with the link handle created once, outside the timed region"},
-        "gpu_launches": None,
+        "gpu_launches": launches,
         "clocks": clk,
         "cpu_baseline": cpu,
         "target_32x32x32x64": target,
         "config4_batch": batch,
     }
-    # our kernel launches per step: one resident loop per reliable update, the
-    # update's own kernels (sum, two Dslashes, residual, copy, direction) and the
-    # start's (norm, two Dslashes, residual, two copies)
-    line["gpu_launches"] = 7 * int(np.median(rus)) + 6
     print(json.dumps(line))
     if pg is not None:
         pg.destroy_process_group()
@@ -674,7 +703,8 @@ def run_profile_mixed(args):
         lib.destroy_V("D", x)
     name = {"single": "single-r12" if args.compress else "single"}.get(args.inner, args.inner)
     lib_tuning = (lib.tuning(name), lib.tuning(name, "mdagm"))
-    # K1 / K2 device time inside one more solve (not timed above)
+    # K1 / K2 device time in one more solve with the separate kernels (the
+    # solves above run the resident loop)
     lib.set_kernel_timing(True)
     x = lib.create_V("D", np.zeros_like(src), "even")
     lib.invert("D", L, x, b, MASS, parity="even", max_iter=MAX_ITER, nrestart=NRESTART, resid=RESID)
@@ -809,7 +839,8 @@ def multishift_workload(dims=MS_DIMS, reps=2, which=None, compress=True, cpu_bas
             d["err_vs_fp64"] = rel(x, x64)
             d["speedup_vs_fp64_cg"] = ms64 / ms
         if inner == "single":
-            # per-kernel CUDA-event durations from one more solve (not timed)
+            # per-kernel CUDA-event durations from one more solve with the
+            # separate kernels (the solves above run the resident loop)
             lib.set_kernel_timing(True)
             _, sti, _, _ = cg(inner, 1)
             lib.set_kernel_timing(False)

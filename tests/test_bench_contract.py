@@ -60,3 +60,14 @@ def test_reference_dslash_mode():
     assert d["impl"] == "reference" and d["lattice"] == "8x8x8x8"
     for prec in ("F", "D"):
         assert d[prec]["us"] > 0 and d[prec]["gbs"] > 0
+
+
+def test_launch_count_of_a_mixed_solve():
+    """The count of one solve's launches by the profiler (969 iterations, 10
+    reliable updates): 74 with the resident loop; with the separate kernels four
+    an iteration take the place of the ten loops."""
+    sys.path.insert(0, ROOT)
+    import bench
+
+    assert bench.mixed_solve_launches(969, 10, 10) == 74
+    assert bench.mixed_solve_launches(969, 10, 0) == 64 + 4 * 969
