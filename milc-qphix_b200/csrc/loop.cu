@@ -40,7 +40,7 @@
 // 15.2, 45.5 / 31.2, 143.5 / 130.0; FP32 with 12-real Naik links 27.9 / 11.9,
 // 33.1 / 18.7, 47.3 / 34.9, 133.2 / 127.4; 16-bit links 27.6 / 12.0, 32.5 /
 // 18.4, 42.7 / 30.5, 104.6 / 99.8.  At 8^4 the barriers are half of the
-// iteration; at 24^3x48 the Dslash phases run at 5.6 TB/s of DRAM with 45 %
+// iteration; at 24^3x48 (12-real) the loop runs at 5.6 TB/s of DRAM with 32 %
 // of the issue slots used, waiting for loads and at the groups' barriers.
 #include <algorithm>
 #include <cstdlib>
@@ -61,9 +61,17 @@ constexpr int kLoopMaxBlocks = 256;         // partial sums per buffer
 // eight_parts: largest lattice (sites per parity) whose Dslash is split into
 // eight parts a site instead of four.  Eight make the chain of loads one stage
 // long, four halve the instructions spent on indices and on the combination.
-// us per iteration with eight / four: 8^4 FP64 11.9 / 14.0, FP32 11.9 / 13.6;
-// 12^3x24 (20736 sites) FP64 22.2 / 23.8, FP32 19.6 / 15.9; 24^3x48 16-bit
-// links 109.5 / 101.3, FP64 271 / 265.
+// The lines are where a lattice fills one round (FP32: 148 SMs x 4 groups x 32
+// sites = 18944) and three rounds (FP64: 148 x 2 x 32 = 9472 each) of
+// eight-part groups; between whole rounds either form can be ahead, by 8 % at
+// most.  us per iteration with eight / four (four phases, 10368, 18432, 20736,
+// 24576 and 30720 sites): FP64 16.6 / 15.4, 17.7 / 17.3, 21.2 / 23.3, 21.4 /
+// 23.0, 26.2 / 25.5; FP32 12.5 / 13.5, 14.9 / 15.1, 18.0 / 16.4, 19.2 / 17.9,
+// 18.9 / 17.2; 12-real 16.9 / 17.1, 18.6 / 17.5, 21.6 / 18.1, 21.9 / 18.9, 23.6
+// / 21.5; 16-bit vectors 17.6 / 16.9, 18.7 / 17.6, 22.8 / 18.5, 23.3 / 19.7,
+// 25.2 / 22.3.  4096 sites: FP64 11.7 / 12.7, FP32 11.4 / 12.6; 24^3x48: 16-bit
+// links 109.5 / 101.3, FP64 271 / 265.  (The eight-part 12- and 13-real forms
+// spill about 90 bytes a thread, the mirrored 13-real one 52.)
 template <typename SV> struct LoopThreads {
     static constexpr int value = 1024, eight_parts = 18944;
 };
@@ -523,9 +531,10 @@ template <> struct FlatWord<double> {
     static __device__ __forceinline__ double2 make(const double v[2]) { return make_double2(v[0], v[1]); }
 };
 
-// The flat phases handle two words of every vector per thread at a time, all
-// loads first: one at a time they ran at the latency of a load per 16 bytes
-// and thread.
+// phase_residual and phase_direction handle two words of every vector per
+// thread at a time, all loads first: one at a time they ran at the latency of a
+// load per 16 bytes and thread.  (The shifts' phases, and k_small_loop, where a
+// thread has one word or none, take one.)
 
 // r += s ttt: |r|^2 of this thread's share
 template <typename SV>
@@ -1071,17 +1080,24 @@ bool solver_loop_run(Prec pv, const LoopRun &q, const Launch &L)
     if (L.halo || dslash_variant_forced() || (e && e[0] == '0')) return false;
     const LinkSet &ls = *q.links;
     // On large lattices the one-thread-per-site Dslash kernels stream the
-    // 16-bit links better than the loop's, and their launches no longer count:
-    // 32^3x64 (1.05 M sites) 291.9 against 309.7 us per iteration, 24^3x48
-    // (0.33 M) 104.6 against 102.4.  With the other storages the loop is the
-    // faster one or equal up to 32^3x64 (FP64 844 / 824, FP32 429 / 412,
-    // 12-real 394.5 / 394.3).
+    // 16-bit links better than the loop's, and their launches no longer count.
+    // us per iteration of the kernels / the loop, FP32 vectors: 24^3x48 (0.33 M
+    // sites) 110.0 / 103.7, 32^3x32 (0.52 M) 163.1 / 158.4, 32^3x48 (0.79 M)
+    // 231.7 / 236.1, 32^3x64 (1.05 M) 298.3 / 314.3; 16-bit vectors 111.4 /
+    // 105.9, 160.0 / 155.7, 228.7 / 228.5, 295.5 / 303.5.  With the other
+    // storages the loop is the faster one or equal: 32^3x64 FP64 847 / 823,
+    // FP32 435 / 415, 12-real 435 / 421; 40^3x64 (2.05 M) 1618 / 1594, 835 /
+    // 811, 817 / 816.
     if (ls.prec == Prec::Half && L.g->vh > kLoopMaxSites16) return false;
     // Updating every shift's two vectors is a stream of its own, which the
-    // kernel's full occupancy moves faster than the loop's one block per SM:
-    // FP64, 12 shifts, 24^3x48 (0.33 M sites) 400.7 against 422.6 us per
-    // iteration, 20^3x40 (0.16 M) 227.0 against 215.3; FP32 218.1 against 208.9
-    // at 24^3x48.
+    // kernel's full occupancy moves faster than the loop's one block per SM, the
+    // more so the more shifts there are.  us per iteration of the kernels / the
+    // loop with 2, 4, 8 and 12 shifts: FP64 20^3x40 (0.16 M sites) 160 / 139,
+    // 173 / 157, 204 / 190, 232 / 219; 24^3x32 (0.22 M) 204 / 191, 224 / 214,
+    // 255 / 252, 285 / 289; 24^3x48 (0.33 M) 294 / 282, 319 / 311, 365 / 368,
+    // 409 / 425.  FP32 24^3x48 158 / 142, 171 / 159, 199 / 186, 226 / 210;
+    // 32^3x32 (0.52 M) 240 / 224, 266 / 245, 302 / 282, 335 / 317: the FP32 line
+    // is below where the two would cross.
     if (q.mode == kLoopMs && L.g->vh > (pv == Prec::Double ? 200000 : 400000)) return false;
     if (pv == Prec::Double && ls.prec == Prec::Double) {
         if (q.mode == kLoopCg) return launch<double, double, kLoopCg>(q, L);
