@@ -2,6 +2,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <system_error>
 #include <thread>
 
 #include "context.h"
@@ -87,6 +88,21 @@ void make_staging(Context &c)
     }
 }
 
+// f(0) .. f(n - 1), each in a thread of its own; where the system refuses a
+// thread, the caller does what is left.
+template <typename F>
+void run_workers(int n, F f)
+{
+    std::vector<std::thread> th;
+    th.reserve(n);
+    try {
+        for (int w = 0; w < n; ++w) th.emplace_back(f, w);
+    } catch (const std::system_error &) {
+    }
+    for (int w = (int)th.size(); w < n; ++w) f(w);
+    for (auto &t : th) t.join();
+}
+
 }  // namespace
 
 void free_staging()
@@ -119,29 +135,25 @@ void h2d_copy(void *dst, const void *src, size_t bytes)
     HostStaging &h = c.staging;
     const int W = h.workers;
     std::atomic<int> failed{0};
-    std::vector<std::thread> th;
-    for (int w = 0; w < W; ++w) {
-        th.emplace_back([&, w] {
-            if (cudaSetDevice(c.device) != cudaSuccess) { failed = 1; return; }
-            // contiguous part of the source, 4 KiB aligned
-            const size_t lo = (bytes * w / W) & ~(size_t)4095, hi = w + 1 == W ? bytes : (bytes * (w + 1) / W) & ~(size_t)4095;
-            int k = 0;
-            for (size_t off = lo; off < hi; off += kStageBytes, ++k) {
-                const size_t n = std::min(kStageBytes, hi - off);
-                const int sl = 2 * w + (k & 1);
-                if (k >= 2 && cudaEventSynchronize(h.done[sl]) != cudaSuccess) { failed = 1; break; }
-                std::memcpy(h.slots[sl], static_cast<const char *>(src) + off, n);
-                if (cudaMemcpyAsync(static_cast<char *>(dst) + off, h.slots[sl], n, cudaMemcpyHostToDevice,
-                                    h.streams[w]) != cudaSuccess ||
-                    cudaEventRecord(h.done[sl], h.streams[w]) != cudaSuccess) {
-                    failed = 1;
-                    break;
-                }
+    run_workers(W, [&](int w) {
+        if (cudaSetDevice(c.device) != cudaSuccess) { failed = 1; return; }
+        // contiguous part of the source, 4 KiB aligned
+        const size_t lo = (bytes * w / W) & ~(size_t)4095, hi = w + 1 == W ? bytes : (bytes * (w + 1) / W) & ~(size_t)4095;
+        int k = 0;
+        for (size_t off = lo; off < hi; off += kStageBytes, ++k) {
+            const size_t n = std::min(kStageBytes, hi - off);
+            const int sl = 2 * w + (k & 1);
+            if (k >= 2 && cudaEventSynchronize(h.done[sl]) != cudaSuccess) { failed = 1; break; }
+            std::memcpy(h.slots[sl], static_cast<const char *>(src) + off, n);
+            if (cudaMemcpyAsync(static_cast<char *>(dst) + off, h.slots[sl], n, cudaMemcpyHostToDevice,
+                                h.streams[w]) != cudaSuccess ||
+                cudaEventRecord(h.done[sl], h.streams[w]) != cudaSuccess) {
+                failed = 1;
+                break;
             }
-            if (cudaStreamSynchronize(h.streams[w]) != cudaSuccess) failed = 1;
-        });
-    }
-    for (auto &t : th) t.join();
+        }
+        if (cudaStreamSynchronize(h.streams[w]) != cudaSuccess) failed = 1;
+    });
     if (failed) throw Error("host to device copy through pinned staging failed");
 }
 
@@ -163,37 +175,33 @@ void d2h_copy(void *dst, const void *src, size_t bytes)
     HostStaging &h = c.staging;
     const int W = h.workers;
     std::atomic<int> failed{0};
-    std::vector<std::thread> th;
-    for (int w = 0; w < W; ++w) {
-        th.emplace_back([&, w] {
-            if (cudaSetDevice(c.device) != cudaSuccess) { failed = 1; return; }
-            const size_t lo = (bytes * w / W) & ~(size_t)4095, hi = w + 1 == W ? bytes : (bytes * (w + 1) / W) & ~(size_t)4095;
-            // chunk k goes device -> slot k&1 while the host copies chunk k-1 out of the other slot
-            size_t prev_off = 0, prev_n = 0;
-            int k = 0;
-            auto drain = [&](int slot) {
-                if (cudaEventSynchronize(h.done[slot]) != cudaSuccess) { failed = 1; return false; }
-                std::memcpy(static_cast<char *>(dst) + prev_off, h.slots[slot], prev_n);
-                return true;
-            };
-            for (size_t off = lo; off < hi; off += kStageBytes, ++k) {
-                const size_t n = std::min(kStageBytes, hi - off);
-                const int sl = 2 * w + (k & 1);
-                if (cudaMemcpyAsync(h.slots[sl], static_cast<const char *>(src) + off, n, cudaMemcpyDeviceToHost,
-                                    h.streams[w]) != cudaSuccess ||
-                    cudaEventRecord(h.done[sl], h.streams[w]) != cudaSuccess) {
-                    failed = 1;
-                    break;
-                }
-                if (k > 0 && !drain(2 * w + ((k - 1) & 1))) break;
-                prev_off = off;
-                prev_n = n;
+    run_workers(W, [&](int w) {
+        if (cudaSetDevice(c.device) != cudaSuccess) { failed = 1; return; }
+        const size_t lo = (bytes * w / W) & ~(size_t)4095, hi = w + 1 == W ? bytes : (bytes * (w + 1) / W) & ~(size_t)4095;
+        // chunk k goes device -> slot k&1 while the host copies chunk k-1 out of the other slot
+        size_t prev_off = 0, prev_n = 0;
+        int k = 0;
+        auto drain = [&](int slot) {
+            if (cudaEventSynchronize(h.done[slot]) != cudaSuccess) { failed = 1; return false; }
+            std::memcpy(static_cast<char *>(dst) + prev_off, h.slots[slot], prev_n);
+            return true;
+        };
+        for (size_t off = lo; off < hi; off += kStageBytes, ++k) {
+            const size_t n = std::min(kStageBytes, hi - off);
+            const int sl = 2 * w + (k & 1);
+            if (cudaMemcpyAsync(h.slots[sl], static_cast<const char *>(src) + off, n, cudaMemcpyDeviceToHost,
+                                h.streams[w]) != cudaSuccess ||
+                cudaEventRecord(h.done[sl], h.streams[w]) != cudaSuccess) {
+                failed = 1;
+                break;
             }
-            if (!failed && k > 0) drain(2 * w + ((k - 1) & 1));
-            if (cudaStreamSynchronize(h.streams[w]) != cudaSuccess) failed = 1;
-        });
-    }
-    for (auto &t : th) t.join();
+            if (k > 0 && !drain(2 * w + ((k - 1) & 1))) break;
+            prev_off = off;
+            prev_n = n;
+        }
+        if (!failed && k > 0) drain(2 * w + ((k - 1) & 1));
+        if (cudaStreamSynchronize(h.streams[w]) != cudaSuccess) failed = 1;
+    });
     if (failed) throw Error("device to host copy through pinned staging failed");
 }
 
