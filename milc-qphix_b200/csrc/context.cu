@@ -58,13 +58,15 @@ namespace {
 // 2.7-3.3 ms with 12 workers each, 1.2-2.5 with 8.
 constexpr size_t kStageBytes = 2u << 20;
 constexpr unsigned kStageWorkers = 12;
-// The smallest copy that goes through the slots: starting and joining the
-// workers takes 0.15 ms, which pays from 9 MiB up and 12 MiB down.  ms of two
-// copies in one call / through the slots, up and down: 4.5 MiB 0.49 / 0.62
-// and 0.57 / 0.76, 7.5 MiB 0.74 / 0.80 and 0.88 / 0.98, 12 MiB 1.14 / 1.02
-// and 1.34 / 1.23, 15 MiB 1.40 / 1.17 and 1.66 / 1.28.  The first staged copy
-// after QPHIX_init also makes the slots and streams, 45-100 ms.
-constexpr size_t kStageMinBytes = 12u << 20;
+// The smallest copies that go through the slots: starting and joining the
+// workers takes 0.15 ms.  ms of two copies in one call / through the slots.
+// Up, from arrays that are not in the host's caches: 3 MiB 0.68 / 0.59-0.76,
+// 4.5 MiB 0.95 / 0.65, 7.5 MiB 1.50 / 0.90, 12 MiB 2.37 / 1.22 (the same array
+// again: 0.41 / 0.54, 0.55 / 0.62, 0.85 / 0.82, 1.32 / 1.07).  Down: 4.5 MiB
+// 0.65 / 0.68, 7.5 MiB 0.88-1.03 / 0.90-0.98, 9 MiB 1.12-1.21 / 0.97-1.03, 12 MiB
+// 1.57 / 1.15.  The first staged copy after QPHIX_init also makes the slots
+// and streams, 45-100 ms.
+constexpr size_t kStageMinUp = 4u << 20, kStageMinDown = 8u << 20;
 
 void make_staging(Context &c)
 {
@@ -123,7 +125,7 @@ void h2d_copy(void *dst, const void *src, size_t bytes)
     cudaPointerAttributes at{};
     const bool pageable = cudaPointerGetAttributes(&at, src) != cudaSuccess || at.type == cudaMemoryTypeUnregistered;
     cudaGetLastError();  // an unregistered pointer is not an error here
-    if (!pageable || bytes < kStageMinBytes) {
+    if (!pageable || bytes < kStageMinUp) {
         QB_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, c.stream));
         QB_CUDA(cudaStreamSynchronize(c.stream));
         return;
@@ -164,7 +166,7 @@ void d2h_copy(void *dst, const void *src, size_t bytes)
     cudaPointerAttributes at{};
     const bool pageable = cudaPointerGetAttributes(&at, dst) != cudaSuccess || at.type == cudaMemoryTypeUnregistered;
     cudaGetLastError();  // an unregistered pointer is not an error here
-    if (!pageable || bytes < kStageMinBytes) {
+    if (!pageable || bytes < kStageMinDown) {
         QB_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, c.stream));
         QB_CUDA(cudaStreamSynchronize(c.stream));
         return;

@@ -1,6 +1,6 @@
 """GPU: copies of pageable host arrays through the pinned slots.
 
-From 12 MiB a copy is shared out over worker threads.  Where the system refuses
+From 4 MiB up and 8 MiB down a copy is shared out over worker threads.  Where the system refuses
 threads (a process limit), the calling thread does the parts that are left: a
 child process puts a pthread_create that can be told to fail in front of the
 system's.
